@@ -207,6 +207,7 @@ def load_library(path: str = LIB_PATH) -> ctypes.CDLL:
         "wfb_scene_boxes_nested": (i32, [vp, ctypes.POINTER(ctypes.c_int)]),
         "wfb_test_traverse": (i32, [vp, vp, i32, i32, i32, i32, i32, vp]),
         "wfb_test_traverse_wide": (i32, [vp, vp, i32, i32, vp, vp]),
+        "wfb_test_traverse_ordered": (i32, [vp, vp, i32, i32, vp, vp]),
         "wfb_device_facts_get": (i32, [vp]),
         "wfb_renderer_l2_window_bytes": (u64, [vp]),
         "wfb_renderer_width": (i32, [vp]),
@@ -317,6 +318,16 @@ class Scene:
         _check(load_library().wfb_test_traverse_wide(self._h, rays.ctypes.data, int(rays.shape[0]), int(bool(anyhit)),
                                                      hits.ctypes.data, counts.ctypes.data))
         return hits, dict(zip(("fetches", "pops", "retests", "binary_steps"), (int(c) for c in counts)))
+
+    def test_traverse_ordered(self, rays: np.ndarray, anyhit: bool = False):
+        """Host run of the ordered wide traversal (wfb_test_traverse_ordered): hits, and counts {nodes,
+        prims, redone, tree}; `tree` 0 means the tree keeps the preorder traversal."""
+        rays = np.ascontiguousarray(rays, RAY)
+        hits = np.zeros(rays.shape[0], HIT)
+        counts = np.zeros(4, np.int64)
+        _check(load_library().wfb_test_traverse_ordered(self._h, rays.ctypes.data, int(rays.shape[0]), int(bool(anyhit)),
+                                                        hits.ctypes.data, counts.ctypes.data))
+        return hits, dict(zip(("nodes", "prims", "redone", "tree"), (int(c) for c in counts)))
 
     def boxes_nested(self) -> bool:
         """True when the BVH's boxes nest, so closest-hit rays may traverse speculatively."""

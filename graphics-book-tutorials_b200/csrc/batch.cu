@@ -110,14 +110,17 @@ void BatchLauncher::launch(const std::vector<JobSpec>& jobs, const std::vector<J
         return;
     }
     last_launches_ = 2;  // persistent megakernel + film commits
-    bool all_split = n > 0;
-    for (int i = 0; i < n; ++i) all_split = all_split && desc[i].chunks > 1;
+    bool all_split = n > 0, all_wide = n > 0;
+    for (int i = 0; i < n; ++i) {
+        all_split = all_split && desc[i].chunks > 1;
+        all_wide = all_wide && wide_usable(desc[i].s);
+    }
     if (!cfg_.use_graph) {
         launch_megakernel_batch(d_jobs_, d_hdr_, max_jobs_, d_counters_, d_work_, count_rays, cfg_.mk, all_split,
-                                stream);
+                                all_wide, stream);
         return;
     }
-    if (graph_exec_ && (count_rays_in_graph_ != count_rays || split_in_graph_ != all_split)) {
+    if (graph_exec_ && (count_rays_in_graph_ != count_rays || split_in_graph_ != all_split || wide_in_graph_ != all_wide)) {
         cudaGraphExecDestroy(graph_exec_);
         graph_exec_ = nullptr;
     }
@@ -126,7 +129,7 @@ void BatchLauncher::launch(const std::vector<JobSpec>& jobs, const std::vector<J
         cuda_check(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal), "begin capture");
         try {
             launch_megakernel_batch(d_jobs_, d_hdr_, max_jobs_, d_counters_, d_work_, count_rays, cfg_.mk, all_split,
-                                    stream);
+                                    all_wide, stream);
         } catch (...) {
             cudaStreamEndCapture(stream, &graph);
             if (graph) cudaGraphDestroy(graph);
@@ -138,6 +141,7 @@ void BatchLauncher::launch(const std::vector<JobSpec>& jobs, const std::vector<J
         cuda_check(e, "instantiate batch graph");
         count_rays_in_graph_ = count_rays;
         split_in_graph_ = all_split;
+        wide_in_graph_ = all_wide;
     }
     cuda_check(cudaGraphLaunch(graph_exec_, stream), "launch batch graph");
 }

@@ -69,6 +69,7 @@ private:
     cudaGraphExec_t graph_exec_ = nullptr;
     bool count_rays_in_graph_ = false;
     bool split_in_graph_ = false;  // the captured graph runs the all-split kernel variant
+    bool wide_in_graph_ = false;   // and the ordered traversal
 };
 
 // Synchronous batch API (wfb_batch_*): owns the films of its jobs.

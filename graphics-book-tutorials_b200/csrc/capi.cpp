@@ -137,7 +137,7 @@ wfb::LaunchConfig launch_config(const wfb_launch_config* c) {
     need(l.mk.block == 64 || l.mk.block == 128 || l.mk.block == 256, "block must be 64, 128 or 256");
     if (c->occupancy >= 0) l.mk.occupancy = l.wf.occupancy = c->occupancy;
     else if (l.mk.block != 128) l.mk.occupancy = 0;  // the register-cap targets exist for block 128 only
-    need(l.mk.occupancy == 0 || (occupancy_target(l.mk.occupancy) && l.mk.block == 128),
+    need(c->occupancy < 0 || l.mk.occupancy == 0 || (occupancy_target(l.mk.occupancy) && l.mk.block == 128),
          "occupancy target must be 0, 6, 8 or 10 (block 128)");
     need(c->min_active <= 32 && c->leaf_batch <= 32, "min_active and leaf_batch must be in 1..32");
     if (c->min_active > 0) l.mk.min_active = l.wf.min_active = c->min_active;
@@ -284,6 +284,16 @@ int wfb_test_traverse_wide(wfb_scene_t s, const void* rays, int n, int anyhit, v
         need(s && counts && (n == 0 || (rays && hits)), "null argument");
         long long c[4] = {0, 0, 0, 0};
         wfb::traverse_wide_check(s->host, static_cast<const float*>(rays), n, anyhit != 0, static_cast<float*>(hits), c);
+        for (int k = 0; k < 4; ++k) counts[k] = (int64_t)c[k];
+    });
+}
+
+int wfb_test_traverse_ordered(wfb_scene_t s, const void* rays, int n, int anyhit, void* hits, int64_t* counts) {
+    return guarded([&] {
+        need(s && counts && (n == 0 || (rays && hits)), "null argument");
+        long long c[4] = {0, 0, 0, 0};
+        wfb::traverse_ordered_check(s->host, static_cast<const float*>(rays), n, anyhit != 0, static_cast<float*>(hits),
+                                    c);
         for (int k = 0; k < 4; ++k) counts[k] = (int64_t)c[k];
     });
 }

@@ -40,6 +40,8 @@ struct DevScene {
     // 1 when every node's box lies inside the box of each node whose subtree holds it (checked at
     // upload): the condition under which speculative closest-hit traversal is exact (box_step).
     int boxes_nested;
+    // Wide nodes over the same leaves (wide_bvh.cuh); null when the tree does not meet their conditions.
+    const float4* wide;
 };
 
 constexpr int kLeafCountBits = 4;
@@ -182,19 +184,9 @@ WF_HD bool can_box_step(int node, int pend, bool spec) {
     return node >= 0 && (pend == 0 || (spec && node < kNodeHeld));
 }
 
-WF_HD void box_step(const float4* __restrict__ nodes, int n_nodes, const wf::Vec3& o,
-                                         const TravRay& ray, float tmax, int& node, int& pend) {
-    // the whole 32-byte node in one 256-bit load (nodes are 32-byte aligned: a 256-byte aligned array
-    // of 32-byte records); +0.9% on icospheres over two 128-bit loads, the same bits
-    float4 na, nb;
-#if defined(__CUDA_ARCH__)
-    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-        : "=f"(na.x), "=f"(na.y), "=f"(na.z), "=f"(na.w), "=f"(nb.x), "=f"(nb.y), "=f"(nb.z), "=f"(nb.w)
-        : "l"(nodes + 2 * node));
-#else
-    na = nodes[2 * node];
-    nb = nodes[2 * node + 1];
-#endif
+// One box step on the loaded node record {na, nb}.
+WF_HD void box_step_on(const float4& na, const float4& nb, int n_nodes, const wf::Vec3& o, const TravRay& ray,
+                       float tmax, int& node, int& pend) {
     const int skip = f2i(na.w);
     if (!wf::hit_box_minmax(wf::Vec3{na.x, na.y, na.z}, wf::Vec3{nb.x, nb.y, nb.z}, o, ray.inv_d, wf::kRayEps, tmax)) {
         node = skip;
@@ -211,6 +203,22 @@ WF_HD void box_step(const float4* __restrict__ nodes, int n_nodes, const wf::Vec
         }
     }
     if (node >= n_nodes) node = -1;
+}
+
+WF_HD void box_step(const float4* __restrict__ nodes, int n_nodes, const wf::Vec3& o,
+                                         const TravRay& ray, float tmax, int& node, int& pend) {
+    // the whole 32-byte node in one 256-bit load (nodes are 32-byte aligned: a 256-byte aligned array
+    // of 32-byte records); +0.9% on icospheres over two 128-bit loads, the same bits
+    float4 na, nb;
+#if defined(__CUDA_ARCH__)
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(na.x), "=f"(na.y), "=f"(na.z), "=f"(na.w), "=f"(nb.x), "=f"(nb.y), "=f"(nb.z), "=f"(nb.w)
+        : "l"(nodes + 2 * node));
+#else
+    na = nodes[2 * node];
+    nb = nodes[2 * node + 1];
+#endif
+    box_step_on(na, nb, n_nodes, o, ray, tmax, node, pend);
 }
 
 WF_HD void prim_step(const float4* __restrict__ prims, int n_spheres, const wf::Vec3& o,

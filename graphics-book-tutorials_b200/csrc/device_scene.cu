@@ -3,6 +3,7 @@
 // precomputed float equals the one the reference computes per ray.
 #include <algorithm>
 #include <atomic>
+#include <cmath>
 #include <cstring>
 #include <exception>
 #include <functional>
@@ -12,6 +13,7 @@
 #include <string>
 #include <vector>
 #include "engine.hpp"
+#include "wide_bvh.cuh"
 #include "../../include/wfb200.h"
 
 namespace wfb {
@@ -59,6 +61,11 @@ DevScene with_camera(const DevScene& s, const wf::Camera& cam, int width, int he
     v.width = width;
     v.height = height;
     return v;
+}
+
+bool wide_usable(const DevScene& s) {
+    const wf::Vec3& o = s.camera.origin;
+    return s.wide != nullptr && std::fabs(o.x) < kCoordMax && std::fabs(o.y) < kCoordMax && std::fabs(o.z) < kCoordMax;
 }
 
 namespace {
@@ -325,8 +332,14 @@ std::shared_ptr<ResidentScene> upload_scene(const wf::Scene& host) {
     float4* lights = reinterpret_cast<float4*>(stage + off[kLights]);
 
     int nested = 0;
+    std::atomic<int> nested_ok{1}, inner_nodes{0};
     const std::function<void(int, int)> pack_nodes = [&](int lo, int hi) {
-        for (int i = lo; i < hi; ++i) pack_node(host, i, nodes + 2 * i);
+        int inner = 0;
+        for (int i = lo; i < hi; ++i) {
+            pack_node(host, i, nodes + 2 * i);
+            inner += host.nodes[i].prim_count <= 0;
+        }
+        inner_nodes += inner;
     };
     const std::function<void(int, int)> pack_prims = [&](int lo, int hi) {
         for (int j = lo; j < hi; ++j) pack_prim(host, j, prims + 3 * j);
@@ -372,7 +385,6 @@ std::shared_ptr<ResidentScene> upload_scene(const wf::Scene& host) {
     const int threads = (size_t)nn + np + nt > (1u << 16) ? (int)std::min(8u, std::max(1u, std::thread::hardware_concurrency())) : 1;
     std::vector<std::function<void()>> sections;
     add_ranges(sections, nn, 1 << 14, threads, pack_nodes);
-    std::atomic<int> nested_ok{1};
     const std::function<void(int, int)> check_nested = [&](int lo, int hi) {
         if (!boxes_nested_range(host.nodes.data(), nn, lo, hi)) nested_ok = 0;
     };
@@ -389,8 +401,13 @@ std::shared_ptr<ResidentScene> upload_scene(const wf::Scene& host) {
     const size_t n_chunks = (total / 8 + kHashChunkWords - 1) / kHashChunkWords;
     // From the stream-ordered pool (on the legacy stream, which orders the copy, the hash and the
     // read-back below): a scene created per frame reuses the memory of the one before it.
-    cuda_check(cudaMallocAsync(&rs->arena, total + n_chunks * 8, 0), "allocate scene");
-    rs->bytes = total;
+    // Behind the packed parts: the chunk hashes and the wide build's control block (read back together), then
+    // the wide nodes, at most one per internal node.
+    const size_t hash_bytes = align256(n_chunks * 8), ctl_bytes = wide_ctl_bytes();
+    const int wide_capacity = nested ? std::max(1, inner_nodes.load()) : 0;
+    const size_t wide_bytes = (size_t)wide_capacity * kWideFloat4 * sizeof(float4);
+    cuda_check(cudaMallocAsync(&rs->arena, total + hash_bytes + ctl_bytes + wide_bytes, 0), "allocate scene");
+    rs->bytes = total + wide_bytes;
     char* base = static_cast<char*>(rs->arena);
     cuda_check(cudaMemcpyAsync(base, stage, total, cudaMemcpyHostToDevice, 0), "cudaMemcpy scene");
     // Content key: chunk hashes of the arena (in the tail of the same allocation), folded here.
@@ -399,25 +416,43 @@ std::shared_ptr<ResidentScene> upload_scene(const wf::Scene& host) {
     hash_chunks<<<(unsigned)((n_chunks + 255) / 256), 256, 0, 0>>>(
         reinterpret_cast<const unsigned long long*>(base), total / 8, chunk_hash);
     cuda_check(cudaGetLastError(), "hash_chunks launch");
-    std::vector<unsigned long long> hashes(n_chunks);
-    cuda_check(cudaMemcpy(hashes.data(), chunk_hash, n_chunks * 8, cudaMemcpyDeviceToHost), "cudaMemcpy hashes");
+    DevScene& d = rs->dev;
+    d.nodes = reinterpret_cast<const float4*>(base + off[kNodes]);
+    d.n_nodes = nn;
+    d.n_spheres = ns;
+    // The wide tree, built from the arena after its hash was taken (the build tags primitive records).
+    float4* wide = reinterpret_cast<float4*>(base + total + hash_bytes + ctl_bytes);
+    constexpr int kLevels = 12;
+    int levels = 0;
+    if (wide_capacity)
+        levels = launch_wide_build(d, reinterpret_cast<float4*>(base + off[kPrims]), wide, wide_capacity,
+                                   base + total + hash_bytes, 0, kLevels, 0);
+    std::vector<unsigned long long> hashes((hash_bytes + ctl_bytes) / 8);
+    cuda_check(cudaMemcpy(hashes.data(), chunk_hash, hash_bytes + ctl_bytes, cudaMemcpyDeviceToHost), "cudaMemcpy hashes");
+    int n_wide = 0;
+    if (wide_capacity) {
+        unsigned long long* ctl = hashes.data() + hash_bytes / 8;
+        bool finished = false;
+        while (n_wide = wide_build_result(ctl, levels, &finished), !finished) {
+            levels = launch_wide_build(d, nullptr, wide, wide_capacity, base + total + hash_bytes, levels, kLevels, 0);
+            cuda_check(cudaMemcpy(ctl, base + total + hash_bytes, ctl_bytes, cudaMemcpyDeviceToHost), "cudaMemcpy wide build");
+        }
+    }
+    d.wide = n_wide > 0 ? wide : nullptr;
+    hashes.resize(n_chunks);
     uint64_t key = 0x6A09E667F3BCC909ull ^ total;
     for (unsigned long long h : hashes) key = fold(key, h);
     key = mix_key(key, &host.env, sizeof(host.env));
     rs->content_key = mix_key(key, &host.camera, sizeof(host.camera));
 
-    DevScene& d = rs->dev;
-    d.nodes = reinterpret_cast<const float4*>(base + off[kNodes]);
     d.prims = reinterpret_cast<const float4*>(base + off[kPrims]);
     d.spheres = reinterpret_cast<const float4*>(base + off[kSpheres]);
     d.tri_shade = reinterpret_cast<const float4*>(base + off[kTriShade]);
     d.tri_area = reinterpret_cast<const float*>(base + off[kTriArea]);
     d.materials = reinterpret_cast<const float4*>(base + off[kMaterials]);
     d.lights = reinterpret_cast<const float4*>(base + off[kLights]);
-    d.n_spheres = ns;
     d.n_triangles = nt;
     d.n_materials = nm;
-    d.n_nodes = nn;
     d.n_lights = nl;
     d.env = host.env;
     d.camera = wf::make_camera_rig(host.camera, host.width, host.height);

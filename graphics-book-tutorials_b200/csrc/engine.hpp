@@ -52,6 +52,17 @@ uint64_t mix_key(uint64_t h, const void* data, size_t bytes);
 
 // 1 when speculative closest-hit traversal is exact on this BVH (nested boxes; device_scene.cu).
 int check_boxes_nested(const std::vector<wf::BvhNode>& nodes);
+// Device build of the wide tree (wide_build.cu): enqueues the leaf check and the first levels (first_level 0) and
+// `levels` later levels on `stream`, and returns how many of the latter are done; `ctl` is wide_ctl_bytes()
+// of device memory, whose host copy wide_build_result reads: the number of wide nodes, 0 when the tree keeps the preorder
+// traversal; `finished` false when levels are left.
+size_t wide_ctl_bytes();
+int launch_wide_build(const DevScene& s, float4* prims, float4* wide, int capacity, void* ctl, int first_level,
+                      int levels, cudaStream_t stream);
+int wide_build_result(const void* ctl_host, int levels_done, bool* finished);
+// Whether renders of this scene view take the ordered traversal (its tree has wide nodes, and the camera,
+// where rays start, is within the range they cover).
+bool wide_usable(const DevScene& s);
 // Packed records (dev_scene.cuh layout) of node i (2 float4) and prim_order entry j (3 float4);
 // throw on what the traversal cannot use.
 void pack_node(const wf::Scene& host, int i, float4* out);
@@ -70,6 +81,11 @@ void traverse_check(const wf::Scene& host, const float* rays, int n, bool anyhit
 // counts[4]: wide fetches, pops, re-tests after a tmax change, binary box steps of the same rays.
 void traverse_wide_check(const wf::Scene& host, const float* rays, int n, bool anyhit, float* hits,
                          long long* counts);
+// Host run of the ordered traversal (wide_bvh.cuh) on the host-built wide tree; counts[4]: wide nodes,
+// primitive tests, rays handed to the preorder steps, wide nodes in the tree (0: the tree does not qualify,
+// and every ray takes the preorder steps).
+void traverse_ordered_check(const wf::Scene& host, const float* rays, int n, bool anyhit, float* hits,
+                            long long* counts);
 
 // Film download in the GPU-arm convention (mean rgb, luminance variance), resolved on the device;
 // shared by renderers, batches and the server. Ordered after the work already queued on `stream`
@@ -104,12 +120,21 @@ struct PassParams {
 struct MegakernelConfig {
     int block = 128;        // threads per CTA (64, 128 or 256)
     int blocks_per_sm = 0;  // 0: as many as fit
-    int min_active = 16;    // traverse on while at least this many lanes of a warp traverse
+    int min_active = 0;     // traverse on while at least this many lanes of a warp traverse; 0: the default
     int split_chunks = 0;   // work units per pixel; 0: one sample per unit while its buffer fits
-    int occupancy = 10;     // block 128 only: 6, 8 or 10 caps registers for that many CTAs per SM (0: none)
-    int leaf_batch = 12;    // a warp tests primitives once this many lanes hold a pending leaf
-    bool speculate = true;  // lanes holding a pending leaf go on with box steps (box_step)
+    int occupancy = -1;     // block 128 only: 6, 8 or 10 caps registers for that many CTAs per SM (0: none); -1: the default
+    int leaf_batch = 0;     // a warp tests primitives once this many lanes hold a pending leaf; 0: the default
+    bool batch = false;     // launches of many jobs (their default min_active differs)
+    // Trees with wide nodes take the ordered traversal (wide_bvh.cuh), others the preorder one with
+    // lanes that hold a pending leaf going on with box steps (box_step); false: the plain preorder steps.
+    bool speculate = true;
 };
+// `cfg` with its defaults filled in. Preorder traversal hides the latency of its node chase with 10 CTAs per SM;
+// the ordered traversal chases 6x fewer nodes with more state per lane, and is faster at 8 with fewer
+// spills (1280x720x16 on a B200, 10 / 8 / 6 CTAs: icospheres 18.0 / 15.3 / 15.4 ms, heightfield 10.7 / 9.6 / 10.3).
+// Its rays end sooner after one another, so it traverses on with fewer lanes before it shades (min_active
+// 2 / 4 / 8 / 16: icospheres 15.8 / 15.3 / 15.3 / 17.5 ms) and waits for fuller primitive rounds.
+MegakernelConfig with_defaults(const MegakernelConfig& cfg, bool wide);
 // Split mode keeps each path's radiance (3 floats) per (pixel, sample) until the ordered commit;
 // automatic splitting keeps that buffer under kSplitBufferBytes (renders above it run in sub-passes).
 constexpr uint64_t kSplitBufferBytes = 2ull << 30;
@@ -189,11 +214,12 @@ __device__ __forceinline__ int job_of_unit(const JobDesc* jobs, int n_jobs, unsi
 void launch_film_commit_jobs(const JobDesc* d_jobs, const BatchHeader* d_hdr, int max_jobs, cudaStream_t stream);
 // Persistent megakernel over a device job table (unit_begin must be the running sum of units)
 // followed by the split-mode commits of its jobs; max_jobs bounds the job count of any batch
-// replayed through the same launch; all_split: every job has chunks > 1 (the leaner kernel variant).
+// replayed through the same launch; all_split: every job has chunks > 1 (the leaner kernel variant);
+// all_wide: every job's scene takes the ordered traversal.
 // Stream-ordered, no host synchronisation, capturable.
 void launch_megakernel_batch(const JobDesc* d_jobs, const BatchHeader* d_hdr, int max_jobs, DevCounters* counters,
                              unsigned int* work_counter, bool count_rays, const MegakernelConfig& cfg,
-                             bool all_split, cudaStream_t stream);
+                             bool all_split, bool all_wide, cudaStream_t stream);
 
 // ---- wavefront (wavefront.cu) ----
 struct WavefrontConfig {
@@ -209,12 +235,9 @@ struct WavefrontConfig {
 // Launch configuration of a batch or a server: the arm and its knobs.
 struct LaunchConfig {
     wf::GpuMode mode = wf::GpuMode::Megakernel;
-    // Batch launches (many jobs of several scenes, shading state parked like a single render's)
-    // traverse best with a lower min_active than one render of one scene: on the 64-job mix on a
-    // B200, 10 CTAs per SM and min_active 12 took 1,168 ms against 1,206 at 8 CTAs and 16.
     MegakernelConfig mk = [] {
         MegakernelConfig c;
-        c.min_active = 12;
+        c.batch = true;
         return c;
     }();
     WavefrontConfig wf{};

@@ -9,6 +9,7 @@
 #include <cstring>
 #include <vector>
 #include "engine.hpp"
+#include "wide_build.cuh"
 #include "../../include/wfb200.h"
 
 namespace wfb {
@@ -182,6 +183,108 @@ void traverse_wide_check(const wf::Scene& host, const float* rays, int n, bool a
     counts[1] = pops;
     counts[2] = retests;
     counts[3] = binary_steps;
+}
+
+namespace {
+
+// Host build of the wide tree, as wide_build.cu does it; empty when the tree does not qualify.
+std::vector<float4> host_wide(const std::vector<float4>& nodes, int nn, std::vector<float4>& prims, int ns) {
+    for (int i = 0; i < nn; ++i) {
+        const float4 lo = nodes[2 * (size_t)i], hi = nodes[2 * (size_t)i + 1];
+        if (!box_in_range(lo, hi)) return {};
+        const int leaf = f2i(hi.w);
+        if (leaf < 0) continue;
+        for (int k = 0; k < (leaf & kLeafCountMask); ++k) {
+            float4* rec = &prims[3 * ((size_t)(leaf >> kLeafCountBits) + k)];
+            if (!prim_in_box(rec, ns, lo, hi) || f2i(rec[1].w) != 0) return {};
+            rec[1].w = i2f_bits(i + 1);
+        }
+    }
+    std::vector<int> roots{0};
+    std::vector<float4> wide;
+    for (size_t w = 0; w < roots.size(); ++w) {
+        int kids[kWideArity], codes[kWideArity];
+        const int k = wide_children(nodes.data(), nn, roots[w], kids);
+        if (k < 0) return {};
+        for (int j = 0; j < k; ++j) {
+            codes[j] = f2i(nodes[2 * (size_t)kids[j] + 1].w);
+            if (codes[j] < 0) {
+                codes[j] = ~(int)roots.size();
+                roots.push_back(kids[j]);
+            }
+        }
+        wide.resize((size_t)kWideFloat4 * (w + 1));
+        wide_write(nodes.data(), kids, codes, k, &wide[(size_t)kWideFloat4 * w]);
+    }
+    return wide;
+}
+
+struct HostStack {
+    int code[kStackShared + kStackLocal];
+    void push(WideState& s, int c, bool on) {
+        if (!on) return;
+        if (s.sp == kStackShared + kStackLocal) s.redo |= kRedoRay;
+        else code[s.sp++] = c;
+    }
+    int pop(int i) const { return code[i]; }
+};
+
+}  // namespace
+
+void traverse_ordered_check(const wf::Scene& host, const float* rays, int n, bool anyhit, float* hits,
+                            long long* counts) {
+    if (n < 0) throw Error(WFB_ERR_INVALID_ARGUMENT, "bad traversal check arguments");
+    if (host.nodes.empty()) throw Error(WFB_ERR_NOT_FINALIZED, "Scene not finalized (no BVH nodes)");
+    const int nn = (int)host.nodes.size(), np = (int)host.prim_order.size();
+    if (nn >= kNodeHeld) throw Error(WFB_ERR_UNSUPPORTED, "BVH has 2^30 nodes or more");
+    std::vector<float4> nodes(2 * (size_t)nn), prims(3 * (size_t)(np > 0 ? np : 1));
+    for (int i = 0; i < nn; ++i) pack_node(host, i, &nodes[2 * (size_t)i]);
+    for (int j = 0; j < np; ++j) pack_prim(host, j, &prims[3 * (size_t)j]);
+    const int ns = (int)host.spheres.size();
+    std::vector<float4> wide;
+    if (check_boxes_nested(host.nodes)) wide = host_wide(nodes, nn, prims, ns);
+    for (int k = 0; k < 4; ++k) counts[k] = 0;
+    counts[3] = (long long)(wide.size() / kWideFloat4);
+    HostStack stack;
+    for (int k = 0; k < n; ++k) {
+        const float* r = rays + 8 * (size_t)k;
+        const wf::Vec3 o{r[0], r[1], r[2]}, d{r[4], r[5], r[6]};
+        TravRay ray;
+        WideState s;
+        wf::HitRecord h;
+        h.t = r[7];
+        h.prim = -1;
+        h.u = h.v = 0.0f;
+        bool redo = wide.empty();
+        if (!redo) {
+            wide_begin(d, r[7], true, &ray, &s);
+            while (s.cur != 0 || s.pend != 0) {
+                if (s.pend != 0) {
+                    ++counts[1];
+                    wide_prim_step(prims.data(), nodes.data(), ns, o, ray, anyhit, s);
+                } else {
+                    ++counts[0];
+                    wide_node_step(wide.data(), o, ray.inv_d, s, stack);
+                }
+                wide_next(s, stack);
+            }
+            redo = anyhit ? s.rank < 0 && s.redo : !wide_resolve(prims.data(), nodes.data(), o, ray, s, &h);
+            if (!redo && s.rank >= 0) {  // the hit's t, u, v by the reference's primitive test
+                int one = (s.rank << kLeafCountBits) | 1, none = -1;
+                h.t = r[7];
+                prim_step(prims.data(), ns, o, ray, anyhit, none, one, h);
+            }
+        }
+        if (redo) {
+            ++counts[2];
+            exact_trace_body(nodes.data(), nn, prims.data(), ns, o, d, r[7], anyhit, &h);
+        }
+        float* out = hits + 4 * (size_t)k;
+        out[0] = h.t;
+        std::memcpy(&out[1], &h.prim, 4);
+        out[2] = h.u;
+        out[3] = h.v;
+    }
 }
 
 }  // namespace wfb

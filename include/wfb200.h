@@ -231,8 +231,8 @@ typedef struct {
     int use_graph;       /* megakernel: replay one captured CUDA graph per launch shape */
     int block;           /* megakernel: 64, 128 or 256 threads; <= 0: 128 */
     int occupancy;       /* register cap for 0, 6, 8 or 10 CTAs per SM: megakernel (block 128) and
-                            wavefront (128-thread blocks); < 0: 10 */
-    int min_active;      /* 1..32; <= 0: default (megakernel batches and servers 12) */
+                            wavefront (128-thread blocks); < 0: the arm's default */
+    int min_active;      /* 1..32; <= 0: default */
     int leaf_batch;      /* 1..32; <= 0: default (see wfb_renderer_configure) */
     int paths_in_flight; /* wavefront pool slots; <= 0: 16M */
     int split_chunks;    /* megakernel: work units per pixel of each job; <= 0: automatic (one
@@ -355,6 +355,12 @@ int wfb_test_traverse(wfb_scene_t scene, const void* rays, int n, int anyhit, in
  * with that tmax; a node popped after tmax moved is tested again. Rays and hits as in
  * wfb_test_traverse; counts[4]: wide fetches, pops, re-tests, binary box steps of the same rays. */
 int wfb_test_traverse_wide(wfb_scene_t scene, const void* rays, int n, int anyhit, void* hits, int64_t* counts);
+/* Host run of the ordered traversal that renders take on trees with wide nodes (no reference counterpart; needs no
+ * GPU): the device's own steps on a wide tree built as the device builds it. Rays and hits as in
+ * wfb_test_traverse (an any-hit query may report another primitive than preorder traversal, never
+ * another yes or no); counts[4]: wide nodes visited, primitive tests, rays handed to the preorder
+ * steps, wide nodes in the tree (0: the tree does not qualify and every ray takes the preorder steps). */
+int wfb_test_traverse_ordered(wfb_scene_t scene, const void* rays, int n, int anyhit, void* hits, int64_t* counts);
 
 /* ---- allocation-free rendering ---------------------------------------------------------------
  * No counterpart in the reference. For callers that must not allocate device memory on their
