@@ -111,16 +111,20 @@ void BatchLauncher::launch(const std::vector<JobSpec>& jobs, const std::vector<J
     }
     last_launches_ = 2;  // persistent megakernel + film commits
     bool all_split = n > 0, all_wide = n > 0;
+    int wide_nodes = 0;
     for (int i = 0; i < n; ++i) {
         all_split = all_split && desc[i].chunks > 1;
         all_wide = all_wide && wide_usable(desc[i].s);
+        wide_nodes = std::max(wide_nodes, desc[i].s.n_nodes);
     }
+    if (!all_wide) wide_nodes = 0;
+    const int tree = wide_nodes == 0 ? 0 : wide_nodes < kSmallTree ? 1 : 2;  // what of it the launch depends on
     if (!cfg_.use_graph) {
         launch_megakernel_batch(d_jobs_, d_hdr_, max_jobs_, d_counters_, d_work_, count_rays, cfg_.mk, all_split,
-                                all_wide, stream);
+                                wide_nodes, stream);
         return;
     }
-    if (graph_exec_ && (count_rays_in_graph_ != count_rays || split_in_graph_ != all_split || wide_in_graph_ != all_wide)) {
+    if (graph_exec_ && (count_rays_in_graph_ != count_rays || split_in_graph_ != all_split || tree_in_graph_ != tree)) {
         cudaGraphExecDestroy(graph_exec_);
         graph_exec_ = nullptr;
     }
@@ -129,7 +133,7 @@ void BatchLauncher::launch(const std::vector<JobSpec>& jobs, const std::vector<J
         cuda_check(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal), "begin capture");
         try {
             launch_megakernel_batch(d_jobs_, d_hdr_, max_jobs_, d_counters_, d_work_, count_rays, cfg_.mk, all_split,
-                                    all_wide, stream);
+                                    wide_nodes, stream);
         } catch (...) {
             cudaStreamEndCapture(stream, &graph);
             if (graph) cudaGraphDestroy(graph);
@@ -141,7 +145,7 @@ void BatchLauncher::launch(const std::vector<JobSpec>& jobs, const std::vector<J
         cuda_check(e, "instantiate batch graph");
         count_rays_in_graph_ = count_rays;
         split_in_graph_ = all_split;
-        wide_in_graph_ = all_wide;
+        tree_in_graph_ = tree;
     }
     cuda_check(cudaGraphLaunch(graph_exec_, stream), "launch batch graph");
 }

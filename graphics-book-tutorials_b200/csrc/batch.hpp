@@ -69,7 +69,7 @@ private:
     cudaGraphExec_t graph_exec_ = nullptr;
     bool count_rays_in_graph_ = false;
     bool split_in_graph_ = false;  // the captured graph runs the all-split kernel variant
-    bool wide_in_graph_ = false;   // and the ordered traversal
+    int tree_in_graph_ = 0;        // preorder, or ordered over small or larger trees
 };
 
 // Synchronous batch API (wfb_batch_*): owns the films of its jobs.

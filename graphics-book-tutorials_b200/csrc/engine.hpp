@@ -118,31 +118,27 @@ struct PassParams {
 
 // ---- megakernel (megakernel.cu) ----
 struct MegakernelConfig {
-    int block = 128;        // threads per CTA (64, 128 or 256)
+    int block = 128;        // threads per CTA (64, 128 or 256; the ordered traversal's kernel has one shape)
     int blocks_per_sm = 0;  // 0: as many as fit
     int min_active = 0;     // traverse on while at least this many lanes of a warp traverse; 0: the default
     int split_chunks = 0;   // work units per pixel; 0: one sample per unit while its buffer fits
-    int occupancy = -1;     // block 128 only: 6, 8 or 10 caps registers for that many CTAs per SM (0: none); -1: the default
+    int occupancy = -1;     // preorder kernel, block 128: 6, 8 or 10 caps registers for that many CTAs per SM (0: none); -1: 10
     int leaf_batch = 0;     // a warp tests primitives once this many lanes hold a pending leaf; 0: the default
     bool batch = false;     // launches of many jobs (their default min_active differs)
     // Trees with wide nodes take the ordered traversal (wide_bvh.cuh), others the preorder one with
     // lanes that hold a pending leaf going on with box steps (box_step); false: the plain preorder steps.
     bool speculate = true;
 };
-// `cfg` with its defaults filled in. Preorder traversal hides the latency of its node chase with 10 CTAs per SM;
-// the ordered traversal chases 6x fewer nodes with more state per lane, and is faster at 8 with fewer
-// spills (1280x720x16 on a B200, 10 / 8 / 6 CTAs: icospheres 18.0 / 15.3 / 15.4 ms, heightfield 10.7 / 9.6 / 10.3).
-// Its rays end sooner after one another, so it traverses on with fewer lanes before it shades (min_active
-// 2 / 4 / 8 / 16: icospheres 15.8 / 15.3 / 15.3 / 17.5 ms) and waits for fuller primitive rounds.
-MegakernelConfig with_defaults(const MegakernelConfig& cfg, bool wide);
+// `cfg` with its defaults filled in. wide_nodes: 0 for the preorder kernel, else the launch takes the ordered traversal over
+// trees of at most that many preorder nodes.
+constexpr int kSmallTree = 4096;
+MegakernelConfig with_defaults(const MegakernelConfig& cfg, int wide_nodes);
 // Split mode keeps each path's radiance (3 floats) per (pixel, sample) until the ordered commit;
 // automatic splitting keeps that buffer under kSplitBufferBytes (renders above it run in sub-passes).
 constexpr uint64_t kSplitBufferBytes = 2ull << 30;
 inline uint64_t split_buffer_bytes(long long pixels, long long samples) {
     return 3ull * sizeof(float) * (uint64_t)pixels * (uint64_t)samples;
 }
-// Resident threads of the persistent megakernel for this configuration.
-int megakernel_resident_threads(const MegakernelConfig& cfg);
 // Work units per pixel (1 = direct film accumulation; > 1 needs a per-sample buffer).
 int megakernel_split_chunks(int pixels, int sample_count, const MegakernelConfig& cfg);
 
@@ -210,16 +206,21 @@ __device__ __forceinline__ int job_of_unit(const JobDesc* jobs, int n_jobs, unsi
 }
 #endif
 
+// The megakernel over the ordered traversal (megakernel_wide.cu): one job in parameter space, or (job0 null) a device job
+// table. Resets nothing and commits nothing; the callers in megakernel.cu do.
+void launch_megakernel_wide(const JobDesc* job0, const JobDesc* d_jobs, const BatchHeader* d_hdr, DevCounters* counters,
+                            unsigned int* work_counter, const MegakernelConfig& cfg, cudaStream_t stream);
+int megakernel_resident_threads(const MegakernelConfig& cfg);  // of the batch form
 // Split-mode commits of every job of a batch (jobs with chunks > 1), in sample order.
 void launch_film_commit_jobs(const JobDesc* d_jobs, const BatchHeader* d_hdr, int max_jobs, cudaStream_t stream);
 // Persistent megakernel over a device job table (unit_begin must be the running sum of units)
 // followed by the split-mode commits of its jobs; max_jobs bounds the job count of any batch
 // replayed through the same launch; all_split: every job has chunks > 1 (the leaner kernel variant);
-// all_wide: every job's scene takes the ordered traversal.
+// wide_nodes: the largest tree's nodes when every job's scene has wide nodes, else 0.
 // Stream-ordered, no host synchronisation, capturable.
 void launch_megakernel_batch(const JobDesc* d_jobs, const BatchHeader* d_hdr, int max_jobs, DevCounters* counters,
                              unsigned int* work_counter, bool count_rays, const MegakernelConfig& cfg,
-                             bool all_split, bool all_wide, cudaStream_t stream);
+                             bool all_split, int wide_nodes, cudaStream_t stream);
 
 // ---- wavefront (wavefront.cu) ----
 struct WavefrontConfig {

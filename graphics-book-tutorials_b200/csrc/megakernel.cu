@@ -1,5 +1,7 @@
 // Persistent megakernel: one lane per path, register-resident state, one launch per render -- or
-// per batch of render jobs.
+// per batch of render jobs. This one traverses in preorder: it renders the scenes whose tree has no wide
+// nodes (wide_bvh.cuh), counting runs, and renders with speculation switched off. The others run
+// megakernel_wide.cu, launched from here.
 //
 // Replaces megakernel_kernel / run_megakernel_pass (WVM/src/gpu/megakernel.cu:11-104), which
 // launches one thread per pixel per sample, traces each path to completion and synchronises the
@@ -38,7 +40,6 @@
 #include <algorithm>
 #include <type_traits>
 #include "engine.hpp"
-#include "wide_bvh.cuh"
 #include "../../include/wfb200.h"
 
 namespace wfb {
@@ -71,46 +72,11 @@ __device__ __forceinline__ const JobDesc& job_at(const MkArgs& a, int j) {
     return MULTI ? a.jobs[j] : a.job0;
 }
 
-// The preorder steps, as a call: the few rays the ordered traversal does not answer (wide_bvh.cuh). Returns
-// {t, prim bits}.
-__device__ __noinline__ float2 exact_trace(const float4* nodes, int n_nodes, const float4* prims, int n_spheres,
-                                           float ox, float oy, float oz, float dx, float dy, float dz, float tmax,
-                                           int anyhit) {
-    wf::HitRecord h;
-    exact_trace_body(nodes, n_nodes, prims, n_spheres, wf::Vec3{ox, oy, oz}, wf::Vec3{dx, dy, dz}, tmax, anyhit != 0, &h);
-    return make_float2(h.t, __int_as_float(h.prim));
-}
-
-// A lane's stack of nodes: the first entries in shared memory, one column per thread, so that lanes at different depths
-// never meet in a bank; deeper ones in local memory.
-template <int BLOCK>
-struct LaneStack {
-    int* top;
-    int* deep;
-    __device__ __forceinline__ void push(WideState& s, int code, bool on) {
-        if (on) {
-            if (s.sp < kStackShared) {
-                top[s.sp * BLOCK] = code;
-                ++s.sp;
-            } else if (s.sp < kStackShared + kStackLocal) {
-                deep[s.sp - kStackShared] = code;
-                ++s.sp;
-            } else {
-                s.redo |= kRedoRay;
-            }
-        }
-    }
-    __device__ __forceinline__ int pop(int i) const {
-        return i < kStackShared ? top[i * BLOCK] : deep[i - kStackShared];
-    }
-};
-
 // MINB > 1 caps registers so that MINB CTAs fit an SM (__launch_bounds__ minimum blocks).
 // COUNT adds node-visit and primitive-test counters (used by count_rays runs only).
 // SPLIT: every job of the launch is in split mode (chunks > 1), so the per-lane film accumulators
 // of direct mode and their branches are compiled out (5 registers fewer under the register cap).
-// WIDE: every scene of the launch has wide nodes, and rays take the ordered traversal (wide_bvh.cuh).
-template <int BLOCK, bool MULTI, int MINB, bool COUNT, bool SPLIT, bool WIDE>
+template <int BLOCK, bool MULTI, int MINB, bool COUNT, bool SPLIT>
 __global__ void __launch_bounds__(BLOCK, MINB) megakernel_persistent(const MkArgs a) {
     const int lane = threadIdx.x & 31;
     const unsigned total_units = MULTI ? a.hdr->total_units : a.job0.units;
@@ -168,23 +134,11 @@ __global__ void __launch_bounds__(BLOCK, MINB) megakernel_persistent(const MkArg
     // batch launches cache the lane's job BVH; a single job reads it from parameter space
     const float4* jnodes = nullptr;
     const float4* jprims = nullptr;
-    const float4* jwide = nullptr;
     int jn_nodes = 0, jn_spheres = 0;
-    // ordered traversal: lane state and stack (one column per thread; deeper entries in local memory)
-    WideState ws;
-    ws.cur = ws.pend = ws.sp = 0;
-    __shared__ int stack_top[WIDE ? kStackShared * BLOCK : 1];
-    int stack_deep[WIDE ? kStackLocal : 1];
-    LaneStack<BLOCK> stack{stack_top + threadIdx.x, stack_deep};
     unsigned n_ext = 0, n_shadow = 0, n_invalid = 0, n_steps = 0, n_prims = 0;
 
     auto start_ray = [&](int boxes_nested) {
         const int nn = MULTI ? jn_nodes : a.job0.s.n_nodes;
-        if (WIDE) {
-            if (shadow_ray) wide_begin(sh_dir, sh_tmax, nn > 0, &ray, &ws);
-            else wide_begin(ps.ray.d, ps.ray.tmax, nn > 0, &ray, &ws);
-            return;
-        }
         if (shadow_ray) traversal_begin(nn, sh_dir, sh_tmax, &ray, &node, &h);
         else traversal_begin(nn, ps.ray.d, ps.ray.tmax, &ray, &node, &h);
         pend = 0;
@@ -197,8 +151,8 @@ __global__ void __launch_bounds__(BLOCK, MINB) megakernel_persistent(const MkArg
     for (;;) {
         // ================= traversal: rounds of box steps or of primitive steps =================
         for (;;) {
-            const bool in_leaf = WIDE ? ws.pend != 0 : pend != 0;
-            const bool at_box = WIDE ? ws.cur < 0 : can_box_step(node, pend, spec);
+            const bool in_leaf = pend != 0;
+            const bool at_box = can_box_step(node, pend, spec);
             const unsigned pmask = __ballot_sync(kFull, in_leaf);
             const unsigned bmask = __ballot_sync(kFull, at_box);
             const unsigned tmask = pmask | bmask;
@@ -213,17 +167,8 @@ __global__ void __launch_bounds__(BLOCK, MINB) megakernel_persistent(const MkArg
             if (np != 0 && (np >= a.leaf_batch || np >= __popc(bmask))) {
                 if (in_leaf) {
                     if (COUNT) ++n_prims;
-                    if (WIDE) {
-                        wide_prim_step(MULTI ? jprims : a.job0.s.prims, MULTI ? jnodes : a.job0.s.nodes,
-                                       MULTI ? jn_spheres : a.job0.s.n_spheres, ps.ray.o, ray, shadow_ray, ws);
-                        wide_next(ws, stack);
-                    } else if (MULTI) prim_step(jprims, jn_spheres, ps.ray.o, ray, shadow_ray, node, pend, h);
+                    if (MULTI) prim_step(jprims, jn_spheres, ps.ray.o, ray, shadow_ray, node, pend, h);
                     else prim_step(a.job0.s.prims, a.job0.s.n_spheres, ps.ray.o, ray, shadow_ray, node, pend, h);
-                }
-            } else if (WIDE) {
-                if (at_box) {
-                    wide_node_step(MULTI ? jwide : a.job0.s.wide, ps.ray.o, ray.inv_d, ws, stack);
-                    wide_next(ws, stack);
                 }
             } else if (at_box) {
 #pragma unroll
@@ -238,26 +183,10 @@ __global__ void __launch_bounds__(BLOCK, MINB) megakernel_persistent(const MkArg
         }
 
         // ================= shading: lanes whose ray has finished =================
-        if ((WIDE ? ws.cur == 0 && ws.pend == 0 : node < 0 && pend == 0) && pixel >= 0) {
+        if (node < 0 && pend == 0 && pixel >= 0) {
             unpark();
             const JobDesc& J = job_at<MULTI>(a, job);
             const DevScene& s = J.s;
-            if (WIDE) {
-                bool redo;
-                if (shadow_ray) {
-                    h.prim = ws.rank;
-                    redo = ws.rank < 0 && ws.redo;
-                } else {
-                    redo = !wide_resolve(s.prims, s.nodes, ps.ray.o, ray, ws, &h);
-                }
-                if (redo) {
-                    const float2 e = exact_trace(s.nodes, s.n_nodes, s.prims, s.n_spheres, ps.ray.o.x, ps.ray.o.y,
-                                                 ps.ray.o.z, ray.d.x, ray.d.y, ray.d.z,
-                                                 shadow_ray ? ws.best : ps.ray.tmax, shadow_ray);
-                    h.t = e.x;
-                    h.prim = __float_as_int(e.y);
-                }
-            }
             bool path_done = false;
             if (shadow_ray) {
                 ++n_shadow;
@@ -361,7 +290,6 @@ __global__ void __launch_bounds__(BLOCK, MINB) megakernel_persistent(const MkArg
                     if (MULTI) {
                         jnodes = s.nodes;
                         jprims = s.prims;
-                        jwide = s.wide;
                         jn_nodes = s.n_nodes;
                         jn_spheres = s.n_spheres;
                     }
@@ -451,28 +379,28 @@ __global__ void film_commit_jobs(const JobDesc* jobs, const BatchHeader* hdr) {
         commit_pixel(J.film, J.lbuf, p, J.sample_count);
 }
 
-template <int BLOCK, bool MULTI, int MINB, bool COUNT, bool SPLIT, bool WIDE>
+template <int BLOCK, bool MULTI, int MINB, bool COUNT, bool SPLIT>
 int resident_ctas(int blocks_per_sm) {
     int dev = 0, sms = 0, occ = 0;
     cuda_check(cudaGetDevice(&dev), "cudaGetDevice");
     cuda_check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "SM count");
     cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-                   &occ, megakernel_persistent<BLOCK, MULTI, MINB, COUNT, SPLIT, WIDE>, BLOCK, 0),
+                   &occ, megakernel_persistent<BLOCK, MULTI, MINB, COUNT, SPLIT>, BLOCK, 0),
                "occupancy");
     if (blocks_per_sm > 0 && blocks_per_sm < occ) occ = blocks_per_sm;
     if (occ < 1) occ = 1;
     return sms * occ;
 }
 
-template <int BLOCK, bool MULTI, int MINB, bool COUNT, bool SPLIT, bool WIDE>
+template <int BLOCK, bool MULTI, int MINB, bool COUNT, bool SPLIT>
 void launch_block(const MkArgs& args, long long units, int blocks_per_sm, cudaStream_t stream) {
-    long long grid = resident_ctas<BLOCK, MULTI, MINB, COUNT, SPLIT, WIDE>(blocks_per_sm);
+    long long grid = resident_ctas<BLOCK, MULTI, MINB, COUNT, SPLIT>(blocks_per_sm);
     if (units > 0) {
         const long long needed = (units + BLOCK - 1) / BLOCK;
         if (grid > needed) grid = needed;
     }
     if (grid < 1) grid = 1;
-    megakernel_persistent<BLOCK, MULTI, MINB, COUNT, SPLIT, WIDE><<<(unsigned)grid, BLOCK, 0, stream>>>(args);
+    megakernel_persistent<BLOCK, MULTI, MINB, COUNT, SPLIT><<<(unsigned)grid, BLOCK, 0, stream>>>(args);
     cuda_check(cudaGetLastError(), "megakernel launch");
 }
 
@@ -489,37 +417,37 @@ auto dispatch(const MegakernelConfig& cfg, F&& f) {
     return f(std::integral_constant<int, 128>{}, std::integral_constant<int, 1>{});
 }
 
-// `all_split`: every job of the launch has chunks > 1 (selects the SPLIT variant). `wide`: the ordered
-// traversal.
+// `all_split`: every job of the launch has chunks > 1 (selects the SPLIT variant).
 template <bool MULTI>
-void launch_any(const MkArgs& args, long long units, const MegakernelConfig& cfg, bool all_split, bool wide,
+void launch_any(const MkArgs& args, long long units, const MegakernelConfig& cfg, bool all_split,
                 cudaStream_t stream) {
     if (args.count_rays) {  // counting runs use the instrumented 128-thread variant (both modes)
-        launch_block<128, MULTI, 1, true, false, false>(args, units, cfg.blocks_per_sm, stream);
+        launch_block<128, MULTI, 1, true, false>(args, units, cfg.blocks_per_sm, stream);
         return;
     }
     dispatch<MULTI>(cfg, [&](auto block, auto minb) {
         constexpr int B = decltype(block)::value, O = decltype(minb)::value;
-        if (wide) {
-            if (all_split) launch_block<B, MULTI, O, false, true, true>(args, units, cfg.blocks_per_sm, stream);
-            else launch_block<B, MULTI, O, false, false, true>(args, units, cfg.blocks_per_sm, stream);
-        } else {
-            if (all_split) launch_block<B, MULTI, O, false, true, false>(args, units, cfg.blocks_per_sm, stream);
-            else launch_block<B, MULTI, O, false, false, false>(args, units, cfg.blocks_per_sm, stream);
-        }
+        if (all_split) launch_block<B, MULTI, O, false, true>(args, units, cfg.blocks_per_sm, stream);
+        else launch_block<B, MULTI, O, false, false>(args, units, cfg.blocks_per_sm, stream);
         return 0;
     });
 }
 
 }  // namespace
 
-MegakernelConfig with_defaults(const MegakernelConfig& cfg, bool wide) {
+MegakernelConfig with_defaults(const MegakernelConfig& cfg, int wide_nodes) {
     MegakernelConfig c = cfg;
-    if (c.occupancy < 0) c.occupancy = wide ? 8 : 10;
+    const bool wide = wide_nodes > 0;
+    if (c.occupancy < 0) c.occupancy = 10;
+    // Ordered traversal: a ray through a tree of a few thousand nodes is short next to shading, which then waits for
+    // more lanes (cornell36 320x180x16, min_active 4 / 8: 0.642 / 0.673 ms); a longer one is not (icospheres
+    // 1280x720x16: 13.3 / 13.0 ms, heightfield 8.74 / 8.50).
     // Preorder batches (many jobs of several scenes) traverse best with a lower min_active than one render of one
     // scene: on the 64-job mix on a B200, 12 took 1,168 ms against 1,206 at 16.
-    if (c.min_active <= 0) c.min_active = wide ? 6 : cfg.batch ? 12 : 16;
-    if (c.leaf_batch <= 0) c.leaf_batch = wide ? 16 : 12;
+    if (c.min_active <= 0) c.min_active = wide ? (wide_nodes < kSmallTree ? 4 : 8) : cfg.batch ? 12 : 16;
+    // A primitive round costs as much as a node round, so it waits for more lanes than in preorder (16 / 24: icospheres
+    // 13.9 / 13.8 ms).
+    if (c.leaf_batch <= 0) c.leaf_batch = wide ? 24 : 12;
     return c;
 }
 
@@ -527,14 +455,6 @@ void launch_film_commit(const DevFilm& film, const float* lbuf, int count, cudaS
     if (film.pixels <= 0 || count <= 0) return;
     film_commit<<<(film.pixels + 255) / 256, 256, 0, stream>>>(film, lbuf, film.pixels, count);
     cuda_check(cudaGetLastError(), "film commit launch");
-}
-
-int megakernel_resident_threads(const MegakernelConfig& config) {
-    const MegakernelConfig cfg = with_defaults(config, true);
-    return dispatch<false>(cfg, [&](auto block, auto minb) {
-        return decltype(block)::value *
-               resident_ctas<decltype(block)::value, false, decltype(minb)::value, false, true, true>(cfg.blocks_per_sm);
-    });
 }
 
 int megakernel_split_chunks(int pixels, int sample_count, const MegakernelConfig& cfg) {
@@ -570,7 +490,7 @@ int launch_megakernel(const DevScene& s, const DevFilm& film, DevCounters* count
                       float* lbuf, const PassParams& p, const MegakernelConfig& config, int chunks,
                       cudaStream_t stream, KernelTimer* timer) {
     const bool wide = config.speculate && !p.count_rays && wide_usable(s);
-    const MegakernelConfig cfg = with_defaults(config, wide);
+    const MegakernelConfig cfg = with_defaults(config, wide ? s.n_nodes : 0);
     if (p.sample_count <= 0 || film.pixels <= 0) return 0;
     if (chunks > 1 && lbuf == nullptr) throw Error(WFB_ERR_INTERNAL, "split megakernel needs a sample buffer");
     MkArgs args{};
@@ -585,7 +505,8 @@ int launch_megakernel(const DevScene& s, const DevFilm& film, DevCounters* count
     args.speculate = cfg.speculate ? 1 : 0;
     cuda_check(cudaMemsetAsync(work_counter, 0, sizeof(unsigned int), stream), "memset work counter");
     if (timer) timer->begin(stream);
-    launch_any<false>(args, args.job0.units, cfg, args.job0.chunks > 1, wide, stream);
+    if (wide) launch_megakernel_wide(&args.job0, nullptr, nullptr, counters, work_counter, cfg, stream);
+    else launch_any<false>(args, args.job0.units, cfg, args.job0.chunks > 1, stream);
     if (timer) timer->end(stream);
     if (args.job0.chunks > 1) {
         launch_film_commit(film, lbuf, p.sample_count, stream);
@@ -596,9 +517,9 @@ int launch_megakernel(const DevScene& s, const DevFilm& film, DevCounters* count
 
 void launch_megakernel_batch(const JobDesc* d_jobs, const BatchHeader* d_hdr, int max_jobs, DevCounters* counters,
                              unsigned int* work_counter, bool count_rays, const MegakernelConfig& config,
-                             bool all_split, bool all_wide, cudaStream_t stream) {
-    const bool wide = config.speculate && !count_rays && all_wide;
-    const MegakernelConfig cfg = with_defaults(config, wide);
+                             bool all_split, int wide_nodes, cudaStream_t stream) {
+    const bool wide = config.speculate && !count_rays && wide_nodes > 0;
+    const MegakernelConfig cfg = with_defaults(config, wide ? wide_nodes : 0);
     MkArgs args{};
     args.jobs = d_jobs;
     args.hdr = d_hdr;
@@ -609,7 +530,9 @@ void launch_megakernel_batch(const JobDesc* d_jobs, const BatchHeader* d_hdr, in
     args.leaf_batch = cfg.leaf_batch;
     args.speculate = cfg.speculate ? 1 : 0;
     cuda_check(cudaMemsetAsync(work_counter, 0, sizeof(unsigned int), stream), "memset work counter");
-    launch_any<true>(args, 0, cfg, all_split, wide, stream);  // full persistent grid: the unit count lives on the device
+    // full persistent grid: the unit count lives on the device
+    if (wide) launch_megakernel_wide(nullptr, d_jobs, d_hdr, counters, work_counter, cfg, stream);
+    else launch_any<true>(args, 0, cfg, all_split, stream);
     launch_film_commit_jobs(d_jobs, d_hdr, max_jobs, stream);
 }
 

@@ -221,12 +221,18 @@ std::vector<float4> host_wide(const std::vector<float4>& nodes, int nn, std::vec
 
 struct HostStack {
     int code[kStackShared + kStackLocal];
-    void push(WideState& s, int c, bool on) {
-        if (!on) return;
+    void push(WideState& s, int c) {
         if (s.sp == kStackShared + kStackLocal) s.redo |= kRedoRay;
         else code[s.sp++] = c;
     }
-    int pop(int i) const { return code[i]; }
+    void push3(WideState& s, int a, bool pa, int b, bool pb, int c, bool pc) {
+        if (pa) push(s, a);
+        if (pb) push(s, b);
+        if (pc) push(s, c);
+    }
+    void pop(WideState& s) const {
+        if (s.sp > 0) s.cur = code[--s.sp];
+    }
 };
 
 }  // namespace
@@ -257,7 +263,7 @@ void traverse_ordered_check(const wf::Scene& host, const float* rays, int n, boo
         h.u = h.v = 0.0f;
         bool redo = wide.empty();
         if (!redo) {
-            wide_begin(d, r[7], true, &ray, &s);
+            wide_begin(d, r[7], true, 0, &ray, &s);
             while (s.cur != 0 || s.pend != 0) {
                 if (s.pend != 0) {
                     ++counts[1];

@@ -52,6 +52,23 @@ WF_HD Vec3& operator*=(Vec3& a, float k) {
     return a;
 }
 
+// Cosine and sine of one angle (the same cosf and sinf as inline). On the device one out-of-line copy serves every
+// caller: inlined at each of them the two functions are a good part of a kernel's instructions.
+struct CosSin {
+    float c, s;
+};
+#if defined(__CUDACC__)
+static __device__ __noinline__ float2 cos_sin_device(float a) { return make_float2(cosf(a), sinf(a)); }
+#endif
+WF_HD CosSin cos_sin(float a) {
+#if defined(__CUDA_ARCH__)
+    const float2 v = cos_sin_device(a);
+    return {v.x, v.y};
+#else
+    return {cosf(a), sinf(a)};
+#endif
+}
+
 // (x*x' + y*y') + z*z', left to right.
 WF_HD float dot(Vec3 a, Vec3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
 WF_HD Vec3 cross(Vec3 a, Vec3 b) {

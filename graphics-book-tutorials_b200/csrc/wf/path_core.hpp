@@ -179,8 +179,8 @@ WF_HD LightSample sample_light(const S& s, Vec3 from, PathKey key, uint32_t dept
         // Uniform direction on the unit sphere (z = 1 - 2 u1, phi = 2 pi u2).
         const float z = 1.0f - 2.0f * u1;
         const float rxy = sqrtf(fmaxf3(0.0f, 1.0f - z * z));
-        const float phi = 2.0f * kPi * u2;
-        const Vec3 dir{rxy * cosf(phi), rxy * sinf(phi), z};
+        const CosSin phi = cos_sin(2.0f * kPi * u2);
+        const Vec3 dir{rxy * phi.c, rxy * phi.s, z};
         ls.n = dir;
         ls.p = g.a + dir * g.radius;
     } else {
@@ -210,26 +210,31 @@ WF_HD float light_pdf_at_hit(const S& s, int prim, float t, Vec3 dir, Vec3 n_out
 }
 
 // Miss / emission (MIS-weighted after a non-delta bounce) / termination. Returns the material type
-// to shade (kLambert, kMetal, kDielectric) or -1 when the path ends here.
+// to shade (kLambert, kMetal, kDielectric) or -1 when the path ends here; `m` gets the surface's material.
 template <class S>
-WF_HD int classify(const S& s, PathState& ps, const HitRecord& h, int max_depth, Surface* surf) {
+WF_HD int classify(const S& s, PathState& ps, const HitRecord& h, int max_depth, Surface* surf, Material* m) {
     if (h.prim < 0) {
         ps.L += ps.throughput * s.env;
         return -1;
     }
     *surf = make_surface(s, ps.ray, h);
-    const Material m = load_material(s, surf->material);
-    if (m.emission.x > 0.0f || m.emission.y > 0.0f || m.emission.z > 0.0f) {
+    *m = load_material(s, surf->material);
+    if (m->emission.x > 0.0f || m->emission.y > 0.0f || m->emission.z > 0.0f) {
         float w = 1.0f;
         if (!ps.specular && ps.prev_pdf > 0.0f) {
             const float pl = light_pdf_at_hit(s, h.prim, h.t, ps.ray.d, surf->n_out);
             w = power_heuristic(ps.prev_pdf, pl);
         }
-        ps.L += ps.throughput * m.emission * w;
+        ps.L += ps.throughput * m->emission * w;
     }
-    if (m.type == kEmissive) return -1;
+    if (m->type == kEmissive) return -1;
     if (ps.depth >= max_depth) return -1;
-    return m.type;
+    return m->type;
+}
+template <class S>
+WF_HD int classify(const S& s, PathState& ps, const HitRecord& h, int max_depth, Surface* surf) {
+    Material m;
+    return classify(s, ps, h, max_depth, surf, &m);
 }
 
 // Survival probability clamp(max throughput, 0.05, 0.95) from depth 3 on; survivors are reweighted.
@@ -248,62 +253,50 @@ WF_HD void set_next_ray(PathState& ps, Vec3 origin, Vec3 dir) {
     ps.ray.tmax = kInf;
 }
 
-// Lambertian: next-event estimation (the shadow ray is returned, not traced), cosine-weighted
-// scattering, roulette. The caller adds *contrib to ps.L if the shadow ray is unoccluded, before
-// the next classify.
-template <class S>
-WF_HD bool shade_lambert(const S& s, PathState& ps, const Surface& f, Ray* shadow, Vec3* contrib,
-                         int* has_shadow) {
-    const Material m = load_material(s, f.material);
-    const uint32_t d = (uint32_t)ps.depth;
-    *has_shadow = 0;
-    const Vec3 org = f.p + f.n * kRayEps;
-    if (s.n_lights > 0) {
-        const LightSample ls = sample_light(s, org, ps.key, d);
-        if (ls.pdf_solid > 0.0f) {
-            const Vec3 to = ls.p - org;
-            const float dist = length(to);
-            const Vec3 wi = to / dist;
-            const float cos_s = dot(f.n, wi);
-            if (cos_s > 0.0f) {
-                const float pb = cos_s * kInvPi;
-                const float w = power_heuristic(ls.pdf_solid, pb);
-                *contrib = ps.throughput * m.albedo * ls.Le * (cos_s * kInvPi * w / ls.pdf_solid);
-                shadow->o = org;
-                shadow->d = wi;
-                shadow->tmin = kRayEps;
-                shadow->tmax = dist * (1.0f - 1e-3f);
-                *has_shadow = 1;
-            }
-        }
-    }
-    // Cosine-weighted direction by Malley's method (uniform disk lifted to the hemisphere).
-    const float u1 = rng(ps.key, d, kDimBsdfU), u2 = rng(ps.key, d, kDimBsdfV);
-    const float r = sqrtf(u1), phi = 2.0f * kPi * u2;
-    Vec3 t, b;
-    make_basis(f.n, &t, &b);
-    const float z = sqrtf(fmaxf3(0.0f, 1.0f - u1));
-    const Vec3 dir = normalize(t * (r * cosf(phi)) + b * (r * sinf(phi)) + f.n * z);
+// The end of every scattering event: throughput, the next ray from `origin` along `dir` (normalised here), roulette.
+WF_HD bool finish_bounce(PathState& ps, const Material& m, Vec3 n, Vec3 origin, Vec3 dir, bool lambert) {
+    const Vec3 d = normalize(dir);
     ps.throughput = ps.throughput * m.albedo;
-    ps.specular = 0;
-    ps.prev_pdf = dot(dir, f.n) * kInvPi;
+    ps.specular = lambert ? 0 : 1;
+    ps.prev_pdf = lambert ? dot(d, n) * kInvPi : 0.0f;
     ps.depth += 1;
-    set_next_ray(ps, org, dir);
+    set_next_ray(ps, origin, d);
     return russian_roulette(ps);
 }
 
-// Tinted perfect mirror.
+// Lambertian, next-event estimation: the shadow ray (returned, not traced) and the contribution it carries. The caller
+// adds *contrib to ps.L if the shadow ray is unoccluded, before the next classify.
 template <class S>
-WF_HD bool shade_metal(const S& s, PathState& ps, const Surface& f) {
-    const Material m = load_material(s, f.material);
-    const Vec3 dir = reflect(ps.ray.d, f.n);
-    if (dot(dir, f.n) <= 0.0f) return false;
-    ps.throughput = ps.throughput * m.albedo;
-    ps.specular = 1;
-    ps.prev_pdf = 0.0f;
-    ps.depth += 1;
-    set_next_ray(ps, f.p + f.n * kRayEps, normalize(dir));
-    return russian_roulette(ps);
+WF_HD int lambert_light(const S& s, const PathState& ps, const Surface& f, const Material& m, Vec3 org, Ray* shadow,
+                        Vec3* contrib) {
+    if (s.n_lights <= 0) return 0;
+    const LightSample ls = sample_light(s, org, ps.key, (uint32_t)ps.depth);
+    if (!(ls.pdf_solid > 0.0f)) return 0;
+    const Vec3 to = ls.p - org;
+    const float dist = length(to);
+    const Vec3 wi = to / dist;
+    const float cos_s = dot(f.n, wi);
+    if (!(cos_s > 0.0f)) return 0;
+    const float pb = cos_s * kInvPi;
+    const float w = power_heuristic(ls.pdf_solid, pb);
+    *contrib = ps.throughput * m.albedo * ls.Le * (cos_s * kInvPi * w / ls.pdf_solid);
+    shadow->o = org;
+    shadow->d = wi;
+    shadow->tmin = kRayEps;
+    shadow->tmax = dist * (1.0f - 1e-3f);
+    return 1;
+}
+
+// Cosine-weighted direction by Malley's method (uniform disk lifted to the hemisphere), not normalised.
+WF_HD Vec3 lambert_direction(const PathState& ps, Vec3 n) {
+    const uint32_t d = (uint32_t)ps.depth;
+    const float u1 = rng(ps.key, d, kDimBsdfU), u2 = rng(ps.key, d, kDimBsdfV);
+    const float r = sqrtf(u1);
+    const CosSin phi = cos_sin(2.0f * kPi * u2);
+    Vec3 t, b;
+    make_basis(n, &t, &b);
+    const float z = sqrtf(fmaxf3(0.0f, 1.0f - u1));
+    return t * (r * phi.c) + b * (r * phi.s) + n * z;
 }
 
 // Unpolarised Fresnel reflectance of a smooth dielectric interface; cos_i >= 0 against the
@@ -317,32 +310,57 @@ WF_HD float fresnel_dielectric(float cos_i, float eta_i, float eta_t) {
     return 0.5f * (r_par * r_par + r_perp * r_perp);
 }
 
-// Smooth dielectric: reflect with probability F, otherwise refract (Snell).
-template <class S>
-WF_HD bool shade_dielectric(const S& s, PathState& ps, const Surface& f) {
-    const Material m = load_material(s, f.material);
+// Smooth dielectric: reflect with probability F, otherwise refract (Snell); direction not normalised.
+WF_HD Vec3 dielectric_direction(const PathState& ps, const Surface& f, const Material& m, Vec3* origin) {
     const float eta_i = f.inside ? m.ior : 1.0f;
     const float eta_t = f.inside ? 1.0f : m.ior;
     const float cos_i = clampf(-dot(ps.ray.d, f.n), 0.0f, 1.0f);
     const float F = fresnel_dielectric(cos_i, eta_i, eta_t);
     const float u = rng(ps.key, (uint32_t)ps.depth, kDimDielectric);
-    Vec3 org, dir;
     if (u < F) {
-        dir = reflect(ps.ray.d, f.n);
-        org = f.p + f.n * kRayEps;
-    } else {
-        const float eta = eta_i / eta_t;
-        const float sin2_t = eta * eta * (1.0f - cos_i * cos_i);
-        const float cos_t = sqrtf(fmaxf3(0.0f, 1.0f - sin2_t));
-        dir = ps.ray.d * eta + f.n * (eta * cos_i - cos_t);
-        org = f.p - f.n * kRayEps;
+        *origin = f.p + f.n * kRayEps;
+        return reflect(ps.ray.d, f.n);
     }
-    ps.throughput = ps.throughput * m.albedo;
-    ps.specular = 1;
-    ps.prev_pdf = 0.0f;
-    ps.depth += 1;
-    set_next_ray(ps, org, normalize(dir));
-    return russian_roulette(ps);
+    const float eta = eta_i / eta_t;
+    const float sin2_t = eta * eta * (1.0f - cos_i * cos_i);
+    const float cos_t = sqrtf(fmaxf3(0.0f, 1.0f - sin2_t));
+    *origin = f.p - f.n * kRayEps;
+    return ps.ray.d * eta + f.n * (eta * cos_i - cos_t);
+}
+
+// A scattering event on material `m` of the given type (kLambert: with a light sample, kMetal: tinted perfect mirror,
+// kDielectric). Returns whether the path goes on. One function for all three, so that lanes of different materials
+// share its end.
+template <class S>
+WF_HD bool shade(const S& s, PathState& ps, const Surface& f, const Material& m, int type, Ray* shadow, Vec3* contrib,
+                 int* has_shadow) {
+    *has_shadow = 0;
+    Vec3 org = f.p + f.n * kRayEps, dir;
+    if (type == kLambert) {
+        *has_shadow = lambert_light(s, ps, f, m, org, shadow, contrib);
+        dir = lambert_direction(ps, f.n);
+    } else if (type == kMetal) {
+        dir = reflect(ps.ray.d, f.n);
+        if (dot(dir, f.n) <= 0.0f) return false;
+    } else {
+        dir = dielectric_direction(ps, f, m, &org);
+    }
+    return finish_bounce(ps, m, f.n, org, dir, type == kLambert);
+}
+
+template <class S>
+WF_HD bool shade_lambert(const S& s, PathState& ps, const Surface& f, Ray* shadow, Vec3* contrib, int* has_shadow) {
+    return shade(s, ps, f, load_material(s, f.material), kLambert, shadow, contrib, has_shadow);
+}
+template <class S>
+WF_HD bool shade_metal(const S& s, PathState& ps, const Surface& f) {
+    int none;
+    return shade(s, ps, f, load_material(s, f.material), kMetal, nullptr, nullptr, &none);
+}
+template <class S>
+WF_HD bool shade_dielectric(const S& s, PathState& ps, const Surface& f) {
+    int none;
+    return shade(s, ps, f, load_material(s, f.material), kDielectric, nullptr, nullptr, &none);
 }
 
 // Whole path of one (pixel, sample) over a SceneView: the reference's trace_path

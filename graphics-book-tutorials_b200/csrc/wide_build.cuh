@@ -102,8 +102,8 @@ WF_HD void wide_write(const float4* nodes, const int* kids, const int* codes, in
         }
     }
     auto bits = [](unsigned u) { return i2f_bits((int)u); };
-    out[0] = make_float4(origin[0], origin[1], origin[2], step[0]);
-    out[1] = make_float4(step[1], step[2], bits(lo_q[0]), bits(hi_q[0]));
+    out[0] = make_float4(origin[0], origin[1], step[0] * 32768.0f, step[1] * 32768.0f);
+    out[1] = make_float4(origin[2], step[2] * 32768.0f, bits(lo_q[0]), bits(hi_q[0]));
     out[2] = make_float4(bits(lo_q[1]), bits(hi_q[1]), bits(lo_q[2]), bits(hi_q[2]));
     int c[kWideArity];
     for (int i = 0; i < kWideArity; ++i) c[i] = i < k ? codes[i] : 0;

@@ -48,8 +48,9 @@ constexpr float kCoordMax = 1.099511627776e12f;
 
 // A wide node is 4 float4 (64 B, two 32-byte loads): a grid (origin, step per axis) and the planes of up to 4 child
 // boxes on it, 8 bits each, child k's in byte k:
-//   {origin.x, origin.y, origin.z, step.x} {step.y, step.z, lo.x[4], hi.x[4]}
+//   {origin.x, origin.y, step.x, step.y} {origin.z, step.z, lo.x[4], hi.x[4]}
 //   {lo.y[4], hi.y[4], lo.z[4], hi.z[4]} {code}[4]
+// (the steps stored times 2^15, see plane_of)
 // code: 0 none, > 0 a leaf (its leaf encoding, start * 16 + count), < 0 ~(wide node index).
 // A plane q lies at origin + q * step. Icospheres: 80K nodes, 5.1 MB, where the preorder nodes are 10.4 MB.
 constexpr int kWideFloat4 = 4;
@@ -57,7 +58,8 @@ constexpr int kWideArity = 4;
 constexpr int kWideMaxLevels = 96;  // a deeper wide tree keeps the preorder traversal
 constexpr float kPlaneMargin = 1.0f / 64.0f;
 
-// Stack entries per lane kept in shared memory; deeper ones go to the lane's local memory.
+// Stack entries per lane kept in shared memory; deeper ones go to the lane's local memory (on icospheres 1 ray in 6,000
+// holds more than 15, none more than 18).
 constexpr int kStackShared = 16;
 constexpr int kStackLocal = 32;
 
@@ -75,18 +77,20 @@ WF_HD bool wide_ray(const TravRay& ray) {
 // (kRedoTie: another hit as near as the best one; kRedoRay: the ray itself is not for this traversal).
 enum : int { kRedoTie = 1, kRedoRay = 2 };
 struct WideState {
-    int cur, pend, sp, rank;
+    int cur, pend;
+    int sp, base;  // stack position, and where it is empty (both in the stack's own units)
+    int rank;
     float best;
     int redo;
 };
 
-WF_HD void wide_begin(wf::Vec3 d, float tmax, bool has_nodes, TravRay* ray, WideState* s) {
+WF_HD void wide_begin(wf::Vec3 d, float tmax, bool has_nodes, int stack_base, TravRay* ray, WideState* s) {
     ray->d = d;
     ray->inv_d = wf::Vec3{1.0f / d.x, 1.0f / d.y, 1.0f / d.z};
     const bool fit = wide_ray(*ray);
     s->cur = has_nodes && fit ? ~0 : 0;
     s->pend = 0;
-    s->sp = 0;
+    s->sp = s->base = stack_base;
     s->rank = -1;
     s->best = tmax;
     s->redo = fit ? 0 : kRedoRay;
@@ -94,13 +98,14 @@ WF_HD void wide_begin(wf::Vec3 d, float tmax, bool has_nodes, TravRay* ray, Wide
 
 // The lane's next node: `cur` stays while it is usable; a leaf becomes the pending one when none is; an
 // empty `cur` is refilled from the stack.
+#pragma nv_exec_check_disable
 template <class Stack>
-WF_HD void wide_next(WideState& s, const Stack& stack) {
-    if (s.cur == 0 && s.sp > 0) s.cur = stack.pop(--s.sp);
+WF_HD void wide_next(WideState& s, Stack& stack) {
+    if (s.cur == 0) stack.pop(s);
     if (s.cur > 0 && s.pend == 0) {
         s.pend = s.cur;
         s.cur = 0;
-        if (s.sp > 0) s.cur = stack.pop(--s.sp);
+        stack.pop(s);
     }
 }
 
@@ -118,24 +123,47 @@ WF_HD float plane_of(unsigned bytes) {
 #endif
 }
 
+// {a.x * b.x + c.x, a.y * b.y + c.y}: one packed instruction on the device.
+WF_HD float2 fma2(float2 a, float2 b, float2 c) {
+#if defined(__CUDA_ARCH__)
+    float2 d;
+    asm("{\n\t.reg .b64 a, b, c, d;\n\t"
+        "mov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tmov.b64 c, {%6, %7};\n\t"
+        "fma.rn.f32x2 d, a, b, c;\n\tmov.b64 {%0, %1}, d;\n\t}"
+        : "=f"(d.x), "=f"(d.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    return d;
+#else
+    return make_float2(fmaf(a.x, b.x, c.x), fmaf(a.y, b.y, c.y));
+#endif
+}
+
 WF_HD unsigned f2u(float f) { return (unsigned)f2i(f); }
 
-// Entry distance of child K's box, infinite when the box is missed. `near`/`far`: the plane bytes by the direction's
-// sign. With a = step / d and b = (origin - o) / d, plane q is met at q a + b = (1 + q 2^-15) (2^15 a) + (b - 2^15 a),
-// whose rounding error is below 2^-22 of the distance plus 0.0021 of a step.
+// A ray against a node's grid: with a = step / d and b = (origin - o) / d, plane q is met at q a + b = (1 + q 2^-15)
+// (2^15 a) + (b - 2^15 a), whose rounding error is below 2^-22 of the distance plus 0.0021 of a step. Plane bytes are
+// chosen by the direction's sign.
+struct WideGrid {
+    unsigned near_x, near_y, near_z, far_x, far_y, far_z;
+    float2 a_xy, b_xy, a_zz, b_zz;
+    float limit;
+};
+
+// Entry distance of child K's box, infinite when the box is missed.
 template <int K>
-WF_HD float child_entry(const unsigned (&near)[3], const unsigned (&far)[3], const wf::Vec3& a, const wf::Vec3& b,
-                        float limit) {
-    const float t0 = fmaxf(fmaxf(fmaf(plane_of<K>(near[0]), a.x, b.x), fmaf(plane_of<K>(near[1]), a.y, b.y)),
-                           fmaxf(fmaf(plane_of<K>(near[2]), a.z, b.z), wf::kRayEps));
-    const float t1 = fminf(fminf(fmaf(plane_of<K>(far[0]), a.x, b.x), fmaf(plane_of<K>(far[1]), a.y, b.y)),
-                           fminf(fmaf(plane_of<K>(far[2]), a.z, b.z), limit));
+WF_HD float child_entry(const WideGrid& g) {
+    const float2 n = fma2(make_float2(plane_of<K>(g.near_x), plane_of<K>(g.near_y)), g.a_xy, g.b_xy);
+    const float2 f = fma2(make_float2(plane_of<K>(g.far_x), plane_of<K>(g.far_y)), g.a_xy, g.b_xy);
+    const float2 z = fma2(make_float2(plane_of<K>(g.near_z), plane_of<K>(g.far_z)), g.a_zz, g.b_zz);
+    const float t0 = fmaxf(fmaxf(n.x, n.y), fmaxf(z.x, wf::kRayEps));
+    const float t1 = fminf(fminf(f.x, f.y), fminf(z.y, g.limit));
     return t0 <= t1 * kBoxSlack ? t0 : INFINITY;
 }
 
 // The lane's wide node: its children are tested together; the nearest one that is met becomes `cur`, the others go
-// on the stack in slot order. Neither a full sort nor entry distances on the stack (to drop entries behind a nearer
+// on the stack. Neither a full sort nor entry distances on the stack (to drop entries behind a nearer
 // hit when they come up) pay: they save 1% and 5-12% of the nodes.
+#pragma nv_exec_check_disable
 template <class Stack>
 WF_HD void wide_node_step(const float4* __restrict__ wide, const wf::Vec3& o, const wf::Vec3& inv, WideState& s,
                           Stack& stack) {
@@ -155,22 +183,36 @@ WF_HD void wide_node_step(const float4* __restrict__ wide, const wf::Vec3& o, co
     q3 = n[3];
 #endif
     const bool sx = inv.x < 0.0f, sy = inv.y < 0.0f, sz = inv.z < 0.0f;
-    const unsigned near[3] = {f2u(sx ? q1.w : q1.z), f2u(sy ? q2.y : q2.x), f2u(sz ? q2.w : q2.z)};
-    const unsigned far[3] = {f2u(sx ? q1.z : q1.w), f2u(sy ? q2.x : q2.y), f2u(sz ? q2.z : q2.w)};
-    const wf::Vec3 a{q0.w * inv.x * 32768.0f, q1.x * inv.y * 32768.0f, q1.y * inv.z * 32768.0f};
-    const wf::Vec3 b{(q0.x - o.x) * inv.x - a.x, (q0.y - o.y) * inv.y - a.y, (q0.z - o.z) * inv.z - a.z};
-    const float limit = s.best * kCullSlack;
-    const float t0 = child_entry<0>(near, far, a, b, limit), t1 = child_entry<1>(near, far, a, b, limit);
-    const float t2 = child_entry<2>(near, far, a, b, limit), t3 = child_entry<3>(near, far, a, b, limit);
-    const int c0 = f2i(q3.x), c1 = f2i(q3.y), c2 = f2i(q3.z), c3 = f2i(q3.w);
-    const float tm = fminf(fminf(t0, t1), fminf(t2, t3));
-    // the nearest: the last slot whose entry is the smallest
-    const bool n3 = t3 == tm, n2 = t2 == tm && !n3, n1 = t1 == tm && !n3 && !n2, n0 = !n1 && !n2 && !n3;
-    s.cur = tm < INFINITY ? (n3 ? c3 : n2 ? c2 : n1 ? c1 : c0) : 0;
-    stack.push(s, c0, t0 < INFINITY && !n0);
-    stack.push(s, c1, t1 < INFINITY && !n1);
-    stack.push(s, c2, t2 < INFINITY && !n2);
-    stack.push(s, c3, t3 < INFINITY && !n3);
+    WideGrid g;
+    g.near_x = f2u(sx ? q1.w : q1.z);
+    g.far_x = f2u(sx ? q1.z : q1.w);
+    g.near_y = f2u(sy ? q2.y : q2.x);
+    g.far_y = f2u(sy ? q2.x : q2.y);
+    g.near_z = f2u(sz ? q2.w : q2.z);
+    g.far_z = f2u(sz ? q2.z : q2.w);
+    g.a_xy = make_float2(q0.z * inv.x, q0.w * inv.y);
+    g.b_xy = fma2(make_float2(q0.x - o.x, q0.y - o.y), make_float2(inv.x, inv.y), make_float2(-g.a_xy.x, -g.a_xy.y));
+    const float az = q1.y * inv.z, bz = fmaf(q1.x - o.z, inv.z, -az);
+    g.a_zz = make_float2(az, az);
+    g.b_zz = make_float2(bz, bz);
+    g.limit = s.best * kCullSlack;
+    // insertion: the nearer of the current choice and the next child stays, the other goes on the stack
+    float tc = child_entry<0>(g);
+    int cur = f2i(q3.x);
+    auto next = [&](float t, int code, int& out) {
+        const bool nearer = t < tc;
+        out = nearer ? cur : code;
+        cur = nearer ? code : cur;
+        const float behind = fmaxf(t, tc);
+        tc = fminf(t, tc);
+        return behind < INFINITY;
+    };
+    int c1, c2, c3;
+    const bool p1 = next(child_entry<1>(g), f2i(q3.y), c1);
+    const bool p2 = next(child_entry<2>(g), f2i(q3.z), c2);
+    const bool p3 = next(child_entry<3>(g), f2i(q3.w), c3);
+    s.cur = tc < INFINITY ? cur : 0;
+    stack.push3(s, c1, p1, c2, p2, c3, p3);
 }
 
 // One primitive of the pending leaf against the ray, as prim_step does. Closest hit: hits up to
@@ -206,11 +248,11 @@ WF_HD void wide_prim_step(const float4* __restrict__ prims, const float4* __rest
             s.rank = rank;
             s.cur = 0;
             s.pend = 0;
-            s.sp = 0;
+            s.sp = s.base;
         }
         return;
     }
-    s.redo = (s.redo & kRedoRay) | (t >= s.best * kTieDown ? kRedoTie : 0);
+    s.redo = (s.redo & ~kRedoTie) | (t >= s.best * kTieDown ? kRedoTie : 0);
     if (t < s.best) {
         s.best = t;
         s.rank = rank;

@@ -176,7 +176,8 @@ int wfb_renderer_render(wfb_renderer_t r, const wfb_render_params* p, wfb_render
 /* GpuRenderer::device_bytes (WVM/src/gpu/gpu_renderer.cu:366-377). */
 uint64_t wfb_renderer_device_bytes(wfb_renderer_t r);
 /* Launch configuration knobs (no reference counterpart; set by the autotuner). Any value < 0
- * keeps the current setting. Megakernel: block 64/128/256 threads, CTAs per SM (0: all that fit),
+ * keeps the current setting. Block and occupancy shape the preorder megakernel; the megakernel of
+ * scenes with wide nodes has one shape. Megakernel: block 64/128/256 threads, CTAs per SM (0: all that fit),
  * the minimum number of traversing lanes per warp before shading runs (1..32), work units per
  * pixel (0: automatic), occupancy target (block 128: 0 none, 6, 8 or 10 CTAs per SM by a register
  * cap), and leaf_batch (1..32): a warp runs a round of primitive tests once this many of its
