@@ -129,11 +129,12 @@ TuneResult autotune(const std::shared_ptr<ResidentScene>& scene, const wf::Camer
         const double samples_w = (double)width * height * pw.sample_count;
         Renderer r(scene, wf::GpuMode::Wavefront);
         r.set_camera(cam, width, height);
-        // stage 1: pool x register cap at the default min_active; stage 2: min_active
+        // stage 1: pool x register cap at one min_active; stage 2: min_active
+        best.wf_min_active = wide_usable(scene->dev) ? 16 : 24;
         const int occs[] = {10, 8};
         for (int pool : pools)
             for (int occ : occs) {
-                r.configure(-1, -1, -1, -1, pool, occ);
+                r.configure(-1, -1, best.wf_min_active, -1, pool, occ);
                 const double ms = measure(r, pw) * samples / samples_w;  // per probe_spp samples
                 best.candidates++;
                 if (ms < wf_ms) {
@@ -142,7 +143,6 @@ TuneResult autotune(const std::shared_ptr<ResidentScene>& scene, const wf::Camer
                     best.wf_occupancy = occ;
                 }
             }
-        best.wf_min_active = WavefrontConfig{}.min_active;
         for (int ma : {16, 24}) {
             r.configure(-1, -1, ma, -1, best.paths_in_flight, best.wf_occupancy);
             const double ms = measure(r, pw) * samples / samples_w;

@@ -103,13 +103,6 @@ void BatchLauncher::launch(const std::vector<JobSpec>& jobs, const std::vector<J
                "upload job table");
     cuda_check(cudaEventRecord(staged_, stream), "cudaEventRecord");
     cuda_check(cudaMemsetAsync(d_counters_, 0, sizeof(DevCounters), stream), "zero counters");
-    if (wf_) {
-        last_launches_ = wf_->run_batch(d_jobs_, d_hdr_, d_counters_, count_rays, stream);
-        launch_film_commit_jobs(d_jobs_, d_hdr_, max_jobs_, stream);
-        ++last_launches_;
-        return;
-    }
-    last_launches_ = 2;  // persistent megakernel + film commits
     bool all_split = n > 0, all_wide = n > 0;
     int wide_nodes = 0;
     for (int i = 0; i < n; ++i) {
@@ -119,6 +112,13 @@ void BatchLauncher::launch(const std::vector<JobSpec>& jobs, const std::vector<J
     }
     if (!all_wide) wide_nodes = 0;
     const int tree = wide_nodes == 0 ? 0 : wide_nodes < kSmallTree ? 1 : 2;  // what of it the launch depends on
+    if (wf_) {
+        last_launches_ = wf_->run_batch(d_jobs_, d_hdr_, d_counters_, count_rays, wide_nodes > 0, stream);
+        launch_film_commit_jobs(d_jobs_, d_hdr_, max_jobs_, stream);
+        ++last_launches_;
+        return;
+    }
+    last_launches_ = 2;  // persistent megakernel + film commits
     if (!cfg_.use_graph) {
         launch_megakernel_batch(d_jobs_, d_hdr_, max_jobs_, d_counters_, d_work_, count_rays, cfg_.mk, all_split,
                                 wide_nodes, stream);

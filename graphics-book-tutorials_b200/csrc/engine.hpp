@@ -226,12 +226,16 @@ void launch_megakernel_batch(const JobDesc* d_jobs, const BatchHeader* d_hdr, in
 struct WavefrontConfig {
     int paths_in_flight = 0;  // path-pool slots; 0: 16M (capped at 64 x pixels)
     int l2_persist = -1;      // pool under a persisting L2 window: -1 when it fits the set-aside, 0 never, 1 always
-    int occupancy = 10;       // register cap for 6, 8 or 10 CTAs of 128 threads per SM (0: none)
+    int occupancy = -1;       // register cap for 6, 8 or 10 CTAs of 128 threads per SM (0: none); -1: the default
     bool suspend_stragglers = true;  // carry the last extension rays of a bounce over to the next
-    int min_active = 24;      // traverse on while at least this many lanes of a warp traverse
-    int leaf_batch = 8;       // a warp tests primitives once this many lanes hold a pending leaf
-    bool speculate = true;    // lanes holding a pending leaf go on with box steps (box_step)
+    int min_active = 0;       // traverse on while at least this many lanes of a warp traverse; 0: the default
+    int leaf_batch = 0;       // a warp tests primitives once this many lanes hold a pending leaf; 0: the default
+    bool speculate = true;    // as in MegakernelConfig
 };
+// The defaults, for the preorder steps and the ordered traversal (its rays are fetched again sooner than they would trace
+// on with few lanes, and its 64-register form is the faster one; icospheres 1280x720x16 at 10 CTAs and 24, 8 and 8, 8:
+// 19.4 / 18.7 ms, with 16 for the primitive rounds 18.5; heightfield 13.3 / 12.5 / 11.7).
+constexpr int kWfOccupancy[2] = {10, 8}, kWfMinActive[2] = {24, 8}, kWfLeafBatch[2] = {8, 16};
 
 // Launch configuration of a batch or a server: the arm and its knobs.
 struct LaunchConfig {

@@ -30,6 +30,7 @@
 #include <mutex>
 #include "engine.hpp"
 #include "queues.cuh"
+#include "wide_lane.cuh"
 #include "wavefront.hpp"
 #include "../../include/wfb200.h"
 
@@ -186,11 +187,22 @@ __device__ bool grid_sync(Control* c, unsigned nblocks, int stage, unsigned long
 // pending leaf and best hit into the pool, slot state 2 -- and leaves; the slot skips this bounce's
 // classify and shading, stays in the active list, and its ray resumes from exactly that state in
 // the next iteration's extend phase. The traversal steps are the same, so the hit is the same.
-template <bool SHADOW, bool MULTI>
+//
+// WIDE: the rays take the ordered traversal (wide_bvh.cuh). Its stragglers are not suspended: its rays are short, and a
+// suspended one would have to take its stack along.
+template <bool SHADOW, bool MULTI, bool WIDE>
 __device__ void traverse_phase(const WfArgs& a, const uint32_t* items, unsigned n, unsigned* cursor,
-                               unsigned long long* n_rays, unsigned* retired = nullptr,
+                               unsigned long long* n_rays, int* stack_words, unsigned* retired = nullptr,
                                unsigned suspend_at = 0xffffffffu) {
     const Pool& P = a.pool;
+    int stack_deep[WIDE ? kStackLocal : 1];
+    LaneStack<kWfBlock> stack{stack_words, stack_deep};
+    WideState ws;
+    ws.cur = ws.pend = ws.redo = 0;
+    ws.rank = -1;
+    ws.best = 0.f;
+    ws.sp = ws.base = threadIdx.x;
+    const float4* wide = a.job0.s.wide;
     // BVH of the lane's current ray: a batch reads its job's from the table at fetch time
     const float4* nodes = a.job0.s.nodes;
     const float4* prims = a.job0.s.prims;
@@ -232,14 +244,19 @@ __device__ void traverse_phase(const WfArgs& a, const uint32_t* items, unsigned 
                         n_nodes = js.n_nodes;
                         n_spheres = js.n_spheres;
                         nested = js.boxes_nested;
+                        wide = js.wide;
                     }
                     const float4 oo = P.ray_o[slot];
                     const float4 d = SHADOW ? P.sh_dir[id] : P.ray_d[id];
                     o = wf::Vec3{oo.x, oo.y, oo.z};
-                    traversal_begin(n_nodes, wf::Vec3{d.x, d.y, d.z}, d.w, &ray, &node, &h);
-                    pend = 0;
-                    spec = a.speculate && (SHADOW || (nested && finite_inv(ray)));
-                    if (!SHADOW && P.alive[slot] == 2u) {  // resume a suspended ray where it stopped
+                    if (WIDE) {
+                        wide_begin(wf::Vec3{d.x, d.y, d.z}, d.w, n_nodes > 0, threadIdx.x, &ray, &ws);
+                    } else {
+                        traversal_begin(n_nodes, wf::Vec3{d.x, d.y, d.z}, d.w, &ray, &node, &h);
+                        pend = 0;
+                        spec = a.speculate && (SHADOW || (nested && finite_inv(ray)));
+                    }
+                    if (!WIDE && !SHADOW && P.alive[slot] == 2u) {  // resume a suspended ray where it stopped
                         const int2 tv = P.trav[slot];
                         const float4 hv = P.hit[slot];
                         node = tv.x;
@@ -260,14 +277,14 @@ __device__ void traverse_phase(const WfArgs& a, const uint32_t* items, unsigned 
         // to fetch); see box_step / prim_step
         unsigned round = 0;
         for (;;) {
-            const bool in_leaf = pend != 0;
-            const bool at_box = can_box_step(node, pend, spec);
+            const bool in_leaf = WIDE ? ws.pend != 0 : pend != 0;
+            const bool at_box = WIDE ? ws.cur < 0 : can_box_step(node, pend, spec);
             const unsigned pm = __ballot_sync(kFull, in_leaf);
             const unsigned bm = __ballot_sync(kFull, at_box);
             const unsigned tm = pm | bm;
             if (tm == 0) break;
             if (__popc(tm) < a.min_active && __ballot_sync(kFull, !(in_leaf || at_box) && !exhausted) != 0) break;
-            if (!SHADOW && (++round & 31u) == 0u && __ballot_sync(kFull, exhausted) != 0) {
+            if (!WIDE && !SHADOW && (++round & 31u) == 0u && __ballot_sync(kFull, exhausted) != 0) {
                 // nothing left to fetch: suspend the warp's rays once most of the phase is done
                 unsigned done = 0;
                 if (lane == 0) done = *(volatile unsigned*)retired;
@@ -291,9 +308,18 @@ __device__ void traverse_phase(const WfArgs& a, const uint32_t* items, unsigned 
             // a single-job launch reads its BVH from parameter space, keeping registers for the ray
             const int np = __popc(pm);
             if (np != 0 && (np >= a.leaf_batch || np >= __popc(bm))) {
-                if (in_leaf) {
+                if (in_leaf && WIDE) {
+                    wide_prim_step(MULTI ? prims : a.job0.s.prims, MULTI ? nodes : a.job0.s.nodes,
+                                   MULTI ? n_spheres : a.job0.s.n_spheres, o, ray, SHADOW, ws);
+                    wide_next(ws, stack);
+                } else if (in_leaf) {
                     if (MULTI) prim_step(prims, n_spheres, o, ray, SHADOW, node, pend, h);
                     else prim_step(a.job0.s.prims, a.job0.s.n_spheres, o, ray, SHADOW, node, pend, h);
+                }
+            } else if (WIDE) {
+                if (at_box) {
+                    wide_node_step(MULTI ? wide : a.job0.s.wide, o, ray.inv_d, ws, stack);
+                    wide_next(ws, stack);
                 }
             } else if (at_box) {
 #pragma unroll
@@ -306,8 +332,19 @@ __device__ void traverse_phase(const WfArgs& a, const uint32_t* items, unsigned 
             }
         }
         // retire finished rays
-        const bool fin = item >= 0 && node < 0 && pend == 0;
-        if (!SHADOW) {
+        const bool fin = item >= 0 && (WIDE ? ws.cur == 0 && ws.pend == 0 : node < 0 && pend == 0);
+        if (WIDE && fin) {  // the hit preorder traversal returns
+            h.prim = ws.rank;
+            const bool redo = SHADOW ? ws.rank < 0 && ws.redo : !wide_resolve(MULTI ? prims : a.job0.s.prims, MULTI ? nodes : a.job0.s.nodes, o, ray, ws, &h);
+            if (redo) {
+                const float2 x = exact_trace(MULTI ? nodes : a.job0.s.nodes, MULTI ? n_nodes : a.job0.s.n_nodes,
+                                             MULTI ? prims : a.job0.s.prims, MULTI ? n_spheres : a.job0.s.n_spheres,
+                                             o.x, o.y, o.z, ray.d.x, ray.d.y, ray.d.z, SHADOW ? ws.best : wf::kInf, SHADOW);
+                h.t = x.x;
+                h.prim = __float_as_int(x.y);
+            }
+        }
+        if (!WIDE && !SHADOW) {
             const unsigned fm = __ballot_sync(kFull, fin);
             if (fm && lane == __ffs(fm) - 1) atomicAdd(retired, (unsigned)__popc(fm));
         }
@@ -334,7 +371,7 @@ __device__ void traverse_phase(const WfArgs& a, const uint32_t* items, unsigned 
 // MINB > 1 caps registers so that MINB CTAs fit an SM (the whole bounce loop is one kernel, so its
 // register count is the largest of any phase's; the traversal phases want the warps more than the
 // shading phases want the registers).
-template <bool MULTI, int MINB>
+template <bool MULTI, int MINB, bool WIDE>
 __global__ void __launch_bounds__(kWfBlock, MINB) wavefront_persistent(const WfArgs a) {
     const Pool& P = a.pool;
     Control* c = P.ctl;
@@ -347,6 +384,7 @@ __global__ void __launch_bounds__(kWfBlock, MINB) wavefront_persistent(const WfA
     __shared__ uint32_t smem[33];
     __shared__ int s_tile;
     __shared__ uint32_t s_prefix;
+    __shared__ int s_stack[WIDE ? kStackShared * kWfBlock : 1];
     unsigned long long t_last = 0;
     if (blockIdx.x == 0 && threadIdx.x == 0) t_last = global_ns();
     unsigned long long n_ext = 0, n_sh = 0;
@@ -487,7 +525,7 @@ __global__ void __launch_bounds__(kWfBlock, MINB) wavefront_persistent(const WfA
 
         // ---------------- E: extension rays ----------------
         // stragglers may be suspended once 95% of a large phase's rays have finished
-        traverse_phase<false, MULTI>(a, next, n, &c->fetch[0], &n_ext, &c->retired,
+        traverse_phase<false, MULTI, WIDE>(a, next, n, &c->fetch[0], &n_ext, s_stack, &c->retired,
                                      a.suspend && n >= 4096 ? n - n / 20 : 0xffffffffu);
         if (!grid_sync(c, nblocks, 0, &t_last, a.wait_ns)) break;
 
@@ -579,7 +617,7 @@ __global__ void __launch_bounds__(kWfBlock, MINB) wavefront_persistent(const WfA
         // ---------------- H: shadow rays ----------------
         const unsigned nsh = min(*(volatile unsigned*)&c->qcount[3], a.qcap);
         if (gtid == 0 && nsh > c->high_water[3]) c->high_water[3] = nsh;
-        traverse_phase<true, MULTI>(a, nullptr, nsh, &c->fetch[1], &n_sh);
+        traverse_phase<true, MULTI, WIDE>(a, nullptr, nsh, &c->fetch[1], &n_sh, s_stack);
         if (!grid_sync(c, nblocks, 5, &t_last, a.wait_ns)) break;
     }
 
@@ -599,13 +637,13 @@ __global__ void __launch_bounds__(kWfBlock, MINB) wavefront_persistent(const WfA
 using WfKernel = void (*)(const WfArgs);
 
 // The compiled register-cap variants: 0 (none), 6, 8 or 10 CTAs of kWfBlock threads per SM.
-template <bool MULTI>
+template <bool MULTI, bool WIDE>
 WfKernel wavefront_kernel(int occupancy) {
     switch (occupancy) {
-        case 6: return wavefront_persistent<MULTI, 6>;
-        case 8: return wavefront_persistent<MULTI, 8>;
-        case 10: return wavefront_persistent<MULTI, 10>;
-        default: return wavefront_persistent<MULTI, 1>;
+        case 6: return wavefront_persistent<MULTI, 6, WIDE>;
+        case 8: return wavefront_persistent<MULTI, 8, WIDE>;
+        case 10: return wavefront_persistent<MULTI, 10, WIDE>;
+        default: return wavefront_persistent<MULTI, 1, WIDE>;
     }
 }
 
@@ -673,9 +711,10 @@ struct WavefrontEngine::State {
     float* lbuf = nullptr;
     size_t lbuf_floats = 0;
     void* acc = nullptr;  // direct-mode film sums per slot (float4 + float), allocated on first use
-    WfKernel kernel = nullptr, kernel_multi = nullptr;  // the register-cap variant of cfg.occupancy
-    int grid = 0;        // co-resident CTAs of the single-render kernel
-    int grid_multi = 0;  // and of the batch kernel
+    // the register-cap variants of cfg.occupancy and their co-resident CTAs: [0] preorder, [1] ordered traversal; for
+    // single renders and for batches
+    WfKernel kernel[2] = {}, kernel_multi[2] = {};
+    int grid[2] = {}, grid_multi[2] = {};
     // L2 residency: an access-policy window over the pool arena on every launch (0 bytes: none)
     size_t window_bytes = 0;
     float hit_ratio = 0.f;
@@ -746,16 +785,22 @@ WavefrontEngine::WavefrontEngine(int pixels, const WavefrontConfig& cfg) : pixel
     cuda_check(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev), "cooperative attribute");
     if (!coop) throw Error(WFB_ERR_UNSUPPORTED, "device does not support cooperative launches");
     cuda_check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "SM count");
-    if (cfg.occupancy != 0 && cfg.occupancy != 6 && cfg.occupancy != 8 && cfg.occupancy != 10)
+    if (cfg.occupancy > 0 && cfg.occupancy != 6 && cfg.occupancy != 8 && cfg.occupancy != 10)
         throw Error(WFB_ERR_INVALID_ARGUMENT, "wavefront occupancy target must be 0, 6, 8 or 10");
-    state_->kernel = wavefront_kernel<false>(cfg.occupancy);
-    state_->kernel_multi = wavefront_kernel<true>(cfg.occupancy);
-    cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, state_->kernel, kWfBlock, 0), "occupancy");
-    if (occ < 1) throw Error(WFB_ERR_UNSUPPORTED, "wavefront kernel does not fit on an SM");
-    state_->grid = sms * occ;
-    cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, state_->kernel_multi, kWfBlock, 0), "occupancy");
-    if (occ < 1) throw Error(WFB_ERR_UNSUPPORTED, "wavefront batch kernel does not fit on an SM");
-    state_->grid_multi = sms * occ;
+    const int cap_preorder = cfg.occupancy >= 0 ? cfg.occupancy : kWfOccupancy[0];
+    const int cap_ordered = cfg.occupancy >= 0 ? cfg.occupancy : kWfOccupancy[1];
+    state_->kernel[0] = wavefront_kernel<false, false>(cap_preorder);
+    state_->kernel[1] = wavefront_kernel<false, true>(cap_ordered);
+    state_->kernel_multi[0] = wavefront_kernel<true, false>(cap_preorder);
+    state_->kernel_multi[1] = wavefront_kernel<true, true>(cap_ordered);
+    for (int w = 0; w < 2; ++w) {
+        cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, state_->kernel[w], kWfBlock, 0), "occupancy");
+        if (occ < 1) throw Error(WFB_ERR_UNSUPPORTED, "wavefront kernel does not fit on an SM");
+        state_->grid[w] = sms * occ;
+        cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, state_->kernel_multi[w], kWfBlock, 0), "occupancy");
+        if (occ < 1) throw Error(WFB_ERR_UNSUPPORTED, "wavefront batch kernel does not fit on an SM");
+        state_->grid_multi[w] = sms * occ;
+    }
     // L2 residency: the pool (every field a bounce reads or writes) under a persisting window when
     // it fits the device's persisting set-aside (auto), or whenever asked (a partial window). Last in
     // the constructor: once the set-aside is counted, nothing can throw, so the destructor's release
@@ -866,6 +911,7 @@ int WavefrontEngine::run(const DevScene& s, const DevFilm& film, DevCounters* co
                          wf::StageTimes* stages, cudaStream_t stream, KernelTimer* timer) {
     if (p.sample_count <= 0 || film.pixels <= 0) return 0;
     State& st = *state_;
+    const int w = cfg_.speculate && wide_usable(s) ? 1 : 0;
     const int chunks = chunks_for(film.pixels, p.sample_count);
     WfArgs a{};
     a.job0 = make_job(s, film, nullptr, p.first_sample, p.sample_count, chunks, p.seed, p.max_depth);
@@ -880,12 +926,12 @@ int WavefrontEngine::run(const DevScene& s, const DevFilm& film, DevCounters* co
     a.pool = st.pool;
     a.capacity = capacity_;
     a.qcap = (p.queue_capacity > 0 && p.queue_capacity < capacity_) ? (uint32_t)p.queue_capacity : (uint32_t)capacity_;
-    a.min_active = cfg_.min_active > 0 ? cfg_.min_active : WavefrontConfig{}.min_active;
-    a.leaf_batch = cfg_.leaf_batch > 0 ? cfg_.leaf_batch : 8;
+    a.min_active = cfg_.min_active > 0 ? cfg_.min_active : kWfMinActive[w];
+    a.leaf_batch = cfg_.leaf_batch > 0 ? cfg_.leaf_batch : kWfLeafBatch[w];
     a.split_shading = p.stage_timing ? 1 : 0;
     a.suspend = cfg_.suspend_stragglers ? 1 : 0;
     a.speculate = cfg_.speculate ? 1 : 0;
-    int launches = launch_pool(st.kernel, a, st.grid, capacity_, counters, p.count_rays, st.window_bytes, st.hit_ratio,
+    int launches = launch_pool(st.kernel[w], a, st.grid[w], capacity_, counters, p.count_rays, st.window_bytes, st.hit_ratio,
                                       stream, timer);
     if (a.job0.chunks > 1) {
         launch_film_commit(film, a.job0.lbuf, p.sample_count, stream);
@@ -908,20 +954,21 @@ int WavefrontEngine::run(const DevScene& s, const DevFilm& film, DevCounters* co
 }
 
 int WavefrontEngine::run_batch(const JobDesc* d_jobs, const BatchHeader* d_hdr, DevCounters* counters,
-                               bool count_rays, cudaStream_t stream) {
+                               bool count_rays, bool all_wide, cudaStream_t stream) {
     reserve_direct();  // a batch may hold direct-mode jobs
+    const int w = cfg_.speculate && all_wide ? 1 : 0;
     WfArgs a{};
     a.jobs = d_jobs;
     a.hdr = d_hdr;
     a.pool = state_->pool;
     a.capacity = capacity_;
     a.qcap = (uint32_t)capacity_;
-    a.min_active = cfg_.min_active > 0 ? cfg_.min_active : WavefrontConfig{}.min_active;
-    a.leaf_batch = cfg_.leaf_batch > 0 ? cfg_.leaf_batch : 8;
+    a.min_active = cfg_.min_active > 0 ? cfg_.min_active : kWfMinActive[w];
+    a.leaf_batch = cfg_.leaf_batch > 0 ? cfg_.leaf_batch : kWfLeafBatch[w];
     a.split_shading = 0;
     a.suspend = cfg_.suspend_stragglers ? 1 : 0;
     a.speculate = cfg_.speculate ? 1 : 0;
-    return launch_pool(state_->kernel_multi, a, state_->grid_multi, capacity_, counters, count_rays, state_->window_bytes,
+    return launch_pool(state_->kernel_multi[w], a, state_->grid_multi[w], capacity_, counters, count_rays, state_->window_bytes,
                              state_->hit_ratio, stream);
 }
 
