@@ -53,7 +53,8 @@ uint64_t mix_key(uint64_t h, const void* data, size_t bytes);
 // 1 when speculative closest-hit traversal is exact on this BVH (nested boxes; device_scene.cu).
 int check_boxes_nested(const std::vector<wf::BvhNode>& nodes);
 // Device build of the wide tree (wide_build.cu): enqueues the leaf check and the first levels (first_level 0) and
-// `levels` later levels on `stream`, and returns how many of the latter are done; `ctl` is wide_ctl_bytes()
+// the later levels (`levels` of them; 0: as many as a tree of this size usually has) on `stream`, and returns how many
+// of the latter are done; `ctl` is wide_ctl_bytes()
 // of device memory, whose host copy wide_build_result reads: the number of wide nodes, 0 when the tree keeps the preorder
 // traversal; `finished` false when levels are left.
 size_t wide_ctl_bytes();
@@ -82,7 +83,7 @@ void traverse_check(const wf::Scene& host, const float* rays, int n, bool anyhit
 void traverse_wide_check(const wf::Scene& host, const float* rays, int n, bool anyhit, float* hits,
                          long long* counts);
 // Host run of the ordered traversal (wide_bvh.cuh) on the host-built wide tree; counts[4]: wide nodes,
-// primitive tests, rays handed to the preorder steps, wide nodes in the tree (0: the tree does not qualify,
+// primitives of the leaves entered, rays handed to the preorder steps, wide nodes in the tree (0: it does not qualify,
 // and every ray takes the preorder steps).
 void traverse_ordered_check(const wf::Scene& host, const float* rays, int n, bool anyhit, float* hits,
                             long long* counts);

@@ -266,15 +266,15 @@ void traverse_ordered_check(const wf::Scene& host, const float* rays, int n, boo
             wide_begin(d, r[7], true, 0, &ray, &s);
             while (s.cur != 0 || s.pend != 0) {
                 if (s.pend != 0) {
-                    ++counts[1];
-                    wide_prim_step(prims.data(), nodes.data(), ns, o, ray, anyhit, s);
+                    counts[1] += s.pend & kLeafCountMask;
+                    wide_leaf_step(prims.data(), ns, o, ray, anyhit, s);
                 } else {
                     ++counts[0];
                     wide_node_step(wide.data(), o, ray.inv_d, s, stack);
                 }
                 wide_next(s, stack);
             }
-            redo = anyhit ? s.rank < 0 && s.redo : !wide_resolve(prims.data(), nodes.data(), o, ray, s, &h);
+            redo = !wide_resolve(prims.data(), nodes.data(), o, ray, anyhit, s, &h);
             if (!redo && s.rank >= 0) {  // the hit's t, u, v by the reference's primitive test
                 int one = (s.rank << kLeafCountBits) | 1, none = -1;
                 h.t = r[7];

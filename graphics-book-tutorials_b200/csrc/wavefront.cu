@@ -309,8 +309,8 @@ __device__ void traverse_phase(const WfArgs& a, const uint32_t* items, unsigned 
             const int np = __popc(pm);
             if (np != 0 && (np >= a.leaf_batch || np >= __popc(bm))) {
                 if (in_leaf && WIDE) {
-                    wide_prim_step(MULTI ? prims : a.job0.s.prims, MULTI ? nodes : a.job0.s.nodes,
-                                   MULTI ? n_spheres : a.job0.s.n_spheres, o, ray, SHADOW, ws);
+                    wide_leaf_step(MULTI ? prims : a.job0.s.prims, MULTI ? n_spheres : a.job0.s.n_spheres, o, ray, SHADOW,
+                                   ws);
                     wide_next(ws, stack);
                 } else if (in_leaf) {
                     if (MULTI) prim_step(prims, n_spheres, o, ray, SHADOW, node, pend, h);
@@ -334,9 +334,7 @@ __device__ void traverse_phase(const WfArgs& a, const uint32_t* items, unsigned 
         // retire finished rays
         const bool fin = item >= 0 && (WIDE ? ws.cur == 0 && ws.pend == 0 : node < 0 && pend == 0);
         if (WIDE && fin) {  // the hit preorder traversal returns
-            h.prim = ws.rank;
-            const bool redo = SHADOW ? ws.rank < 0 && ws.redo : !wide_resolve(MULTI ? prims : a.job0.s.prims, MULTI ? nodes : a.job0.s.nodes, o, ray, ws, &h);
-            if (redo) {
+            if (!wide_resolve(MULTI ? prims : a.job0.s.prims, MULTI ? nodes : a.job0.s.nodes, o, ray, SHADOW, ws, &h)) {
                 const float2 x = exact_trace(MULTI ? nodes : a.job0.s.nodes, MULTI ? n_nodes : a.job0.s.n_nodes,
                                              MULTI ? prims : a.job0.s.prims, MULTI ? n_spheres : a.job0.s.n_spheres,
                                              o.x, o.y, o.z, ray.d.x, ray.d.y, ray.d.z, SHADOW ? ws.best : wf::kInf, SHADOW);

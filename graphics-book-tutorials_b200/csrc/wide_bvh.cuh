@@ -23,7 +23,8 @@
 //    the triangle's plane that still meets the triangle and has another surface in the gap.
 //  * Any-hit queries (shadow rays) have a fixed tmax, so whether a leaf is entered depends on its
 //    box alone: occluded when some leaf whose box passes holds a primitive hit below tmax, in any
-//    order. Exact, with the leaf's own box test run before a hit counts.
+//    order. Exact, with the leaf's own box test run on the hit that ended the query (should it fail, the
+//    preorder steps answer).
 //
 // Conditions on the tree, checked at upload (wide_build.cu): nested boxes, every primitive inside
 // its leaf's box, each prim_order entry in one leaf, finite coordinates below kCoordMax, at most 4
@@ -215,48 +216,47 @@ WF_HD void wide_node_step(const float4* __restrict__ wide, const wf::Vec3& o, co
     stack.push3(s, c1, p1, c2, p2, c3, p3);
 }
 
-// One primitive of the pending leaf against the ray, as prim_step does. Closest hit: hits up to
+// The primitives of the pending leaf against the ray, each as prim_step tests it. Closest hit: hits up to
 // best * kTieUp are seen, so that a tie on either side of the best sets `redo`; a clearly nearer hit
-// clears it again. Any hit: the first hit whose leaf's own box test passes ends the query.
-WF_HD void wide_prim_step(const float4* __restrict__ prims, const float4* __restrict__ nodes, int n_spheres,
-                          const wf::Vec3& o, const TravRay& ray, bool anyhit, WideState& s) {
-    const int rank = s.pend >> kLeafCountBits;
-    const float4* rec = prims + 3 * rank;
-    const float4 q0 = ro_load(rec);
-    const float4 q1 = ro_load(rec + 1);
-    wf::Ray r;
-    r.o = o;
-    r.d = ray.d;
-    r.tmin = wf::kRayEps;
-    r.tmax = anyhit ? s.best : s.best * kTieUp;
-    float t, u, v;
-    bool hit;
-    if (f2i(q0.w) < n_spheres) {
-        hit = wf::hit_sphere_core(wf::Vec3{q0.x, q0.y, q0.z}, q1.x, r, &t);
-    } else {
-        const float4 q2 = ro_load(rec + 2);
-        hit = wf::hit_triangle_core(wf::Vec3{q0.x, q0.y, q0.z}, wf::Vec3{q1.x, q1.y, q1.z},
-                                    wf::Vec3{q2.x, q2.y, q2.z}, r, &t, &u, &v);
-    }
-    s.pend += (1 << kLeafCountBits) - 1;
-    if ((s.pend & kLeafCountMask) == 0) s.pend = 0;
-    if (!hit) return;
-    if (anyhit) {
-        const int leaf = f2i(q1.w) - 1;
-        const float4 a = ro_load(nodes + 2 * leaf), b = ro_load(nodes + 2 * leaf + 1);
-        if (wf::hit_box_minmax(wf::Vec3{a.x, a.y, a.z}, wf::Vec3{b.x, b.y, b.z}, o, ray.inv_d, wf::kRayEps, s.best)) {
-            s.rank = rank;
-            s.cur = 0;
-            s.pend = 0;
-            s.sp = s.base;
+// clears it again. Any hit: the first hit ends the query (wide_resolve runs its leaf's own box test).
+WF_HD void wide_leaf_step(const float4* __restrict__ prims, int n_spheres, const wf::Vec3& o, const TravRay& ray,
+                          bool anyhit, WideState& s) {
+    {
+        const int rank = s.pend >> kLeafCountBits;
+        const float4* rec = prims + 3 * rank;
+        const float4 q0 = ro_load(rec);
+        const float4 q1 = ro_load(rec + 1);
+        wf::Ray r;
+        r.o = o;
+        r.d = ray.d;
+        r.tmin = wf::kRayEps;
+        r.tmax = anyhit ? s.best : s.best * kTieUp;
+        float t, u, v;
+        bool hit;
+        if (f2i(q0.w) < n_spheres) {
+            hit = wf::hit_sphere_core(wf::Vec3{q0.x, q0.y, q0.z}, q1.x, r, &t);
+        } else {
+            const float4 q2 = ro_load(rec + 2);
+            hit = wf::hit_triangle_core(wf::Vec3{q0.x, q0.y, q0.z}, wf::Vec3{q1.x, q1.y, q1.z},
+                                        wf::Vec3{q2.x, q2.y, q2.z}, r, &t, &u, &v);
         }
-        return;
+        s.pend += (1 << kLeafCountBits) - 1;
+        if (hit) {
+            if (anyhit) {
+                s.rank = rank;
+                s.cur = 0;
+                s.pend = 0;
+                s.sp = s.base;
+            } else {
+                s.redo = (s.redo & ~kRedoTie) | (t >= s.best * kTieDown ? kRedoTie : 0);
+                if (t < s.best) {
+                    s.best = t;
+                    s.rank = rank;
+                }
+            }
+        }
     }
-    s.redo = (s.redo & ~kRedoTie) | (t >= s.best * kTieDown ? kRedoTie : 0);
-    if (t < s.best) {
-        s.best = t;
-        s.rank = rank;
-    }
+    if ((s.pend & kLeafCountMask) == 0) s.pend = 0;
 }
 
 // The preorder steps from the ray's start: what the ordered traversal hands over to.
@@ -272,19 +272,19 @@ WF_HD void exact_trace_body(const float4* __restrict__ nodes, int n_nodes, const
     }
 }
 
-// A closest-hit ray at its end: true when the best hit is the one preorder traversal returns (its leaf
-// box is met, and entered by best * kEntryUp); `h` gets it. A miss without `redo` is a miss.
+// A ray at its end: true when what it found is what preorder traversal finds; `h` gets it. Closest hit: the best hit
+// has no tie, and its leaf's box is met, and entered by best * kEntryUp. Any hit: the leaf's box passes with the
+// ray's tmax; else another leaf may hold the hit. A miss without `redo` is a miss.
 WF_HD bool wide_resolve(const float4* __restrict__ prims, const float4* __restrict__ nodes, const wf::Vec3& o,
-                        const TravRay& ray, const WideState& s, wf::HitRecord* h) {
-    if (s.redo) return false;
+                        const TravRay& ray, bool anyhit, const WideState& s, wf::HitRecord* h) {
     h->t = s.best;
     h->prim = -1;
-    if (s.rank < 0) return true;
+    if (s.rank < 0 || (s.redo && !anyhit)) return s.redo == 0;
     h->prim = f2i(ro_load(prims + 3 * s.rank).w);
     const int leaf = f2i(ro_load(prims + 3 * s.rank + 1).w) - 1;
     const float4 a = ro_load(nodes + 2 * leaf), b = ro_load(nodes + 2 * leaf + 1);
     return wf::hit_box_minmax(wf::Vec3{a.x, a.y, a.z}, wf::Vec3{b.x, b.y, b.z}, o, ray.inv_d, wf::kRayEps,
-                              s.best * kEntryUp);
+                              anyhit ? s.best : s.best * kEntryUp);
 }
 
 #endif  // __CUDACC__
