@@ -92,9 +92,10 @@ WF_HD void wide_write(const float4* nodes, const int* kids, const int* codes, in
         const double s = fmax(fmax(extent / 254.0, size * 4.8e-7), 1e-11);
         step[x] = (float)(s * 1.0000002);
         origin[x] = (float)((double)lo - 0.25 * s);
+        const double per_step = 1.0 / (double)step[x];
         for (int i = 0; i < k; ++i) {
-            const double a = ((double)at(nodes[2 * kids[i]]) - (double)origin[x]) / (double)step[x] - kPlaneMargin;
-            const double b = ((double)at(nodes[2 * kids[i] + 1]) - (double)origin[x]) / (double)step[x] + kPlaneMargin;
+            const double a = ((double)at(nodes[2 * kids[i]]) - (double)origin[x]) * per_step - kPlaneMargin;
+            const double b = ((double)at(nodes[2 * kids[i] + 1]) - (double)origin[x]) * per_step + kPlaneMargin;
             const unsigned qa = (unsigned)fmin(fmax(floor(a), 0.0), 255.0);
             const unsigned qb = (unsigned)fmin(fmax(ceil(b), 0.0), 255.0);
             lo_q[x] = (lo_q[x] & ~(255u << (8 * i))) | (qa << (8 * i));
