@@ -149,6 +149,17 @@ void add_ranges(std::vector<std::function<void()>>& fs, int n, int grain, int pa
 
 }  // namespace
 
+StagingLock::StagingLock() {
+    Staging& st = staging();
+    if (!st.mu.try_lock()) return;
+    data = st.p;
+    bytes = st.cap;
+    if (!data) st.mu.unlock();
+}
+StagingLock::~StagingLock() {
+    if (data) staging().mu.unlock();
+}
+
 void pack_node(const wf::Scene& host, int i, float4* out) {
     // {lo, skip} {hi, leaf}
     const int nn = (int)host.nodes.size(), np = (int)host.prim_order.size();

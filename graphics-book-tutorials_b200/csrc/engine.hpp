@@ -88,6 +88,15 @@ void traverse_wide_check(const wf::Scene& host, const float* rays, int n, bool a
 void traverse_ordered_check(const wf::Scene& host, const float* rays, int n, bool anyhit, float* hits,
                             long long* counts);
 
+// The pinned staging of scene uploads, for a short copy of something else: data is null when an upload has it.
+struct StagingLock {
+    char* data = nullptr;
+    size_t bytes = 0;
+    StagingLock();
+    ~StagingLock();
+    StagingLock(const StagingLock&) = delete;
+    StagingLock& operator=(const StagingLock&) = delete;
+};
 // Film download in the GPU-arm convention (mean rgb, luminance variance), resolved on the device;
 // shared by renderers, batches and the server. Ordered after the work already queued on `stream`
 // (null: the calling thread's own stream, for a film whose writers have finished); returns once
@@ -162,10 +171,11 @@ private:
 };
 // Adds samples [first, first + count) of every pixel to `film`. With chunks > 1, `lbuf` must hold
 // 3 * pixels * count floats (per-sample radiance, committed in sample order after the kernel).
-// Returns the number of kernels launched.
+// work_is_zero: the caller has zeroed *work_counter. Returns the number of kernels launched.
 int launch_megakernel(const DevScene& s, const DevFilm& film, DevCounters* counters,
                        unsigned int* work_counter, float* lbuf, const PassParams& p,
-                      const MegakernelConfig& cfg, int chunks, cudaStream_t stream, KernelTimer* timer = nullptr);
+                      const MegakernelConfig& cfg, int chunks, cudaStream_t stream, KernelTimer* timer = nullptr,
+                      bool work_is_zero = false);
 
 // Adds per-(pixel, sample) radiance slots (3 floats, sample-major: sample_slot) to the
 // film sums in ascending sample order (megakernel.cu).

@@ -488,7 +488,7 @@ JobDesc make_job(const DevScene& s, const DevFilm& film, float* lbuf, int first_
 
 int launch_megakernel(const DevScene& s, const DevFilm& film, DevCounters* counters, unsigned int* work_counter,
                       float* lbuf, const PassParams& p, const MegakernelConfig& config, int chunks,
-                      cudaStream_t stream, KernelTimer* timer) {
+                      cudaStream_t stream, KernelTimer* timer, bool work_is_zero) {
     const bool wide = config.speculate && !p.count_rays && wide_usable(s);
     const MegakernelConfig cfg = with_defaults(config, wide ? s.n_nodes : 0);
     if (p.sample_count <= 0 || film.pixels <= 0) return 0;
@@ -503,7 +503,7 @@ int launch_megakernel(const DevScene& s, const DevFilm& film, DevCounters* count
     args.min_active = cfg.min_active;
     args.leaf_batch = cfg.leaf_batch;
     args.speculate = cfg.speculate ? 1 : 0;
-    cuda_check(cudaMemsetAsync(work_counter, 0, sizeof(unsigned int), stream), "memset work counter");
+    if (!work_is_zero) cuda_check(cudaMemsetAsync(work_counter, 0, sizeof(unsigned int), stream), "memset work counter");
     if (timer) timer->begin(stream);
     if (wide) launch_megakernel_wide(&args.job0, nullptr, nullptr, counters, work_counter, cfg, stream);
     else launch_any<false>(args, args.job0.units, cfg, args.job0.chunks > 1, stream);

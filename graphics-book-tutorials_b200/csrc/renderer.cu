@@ -16,6 +16,9 @@ namespace {
 // allocation after the first, where cudaMalloc of a 700 MB sample buffer takes milliseconds.
 constexpr uint64_t kPoolKeepBytes = 8ull << 30;
 
+// The counters' share of the block they and the work counter lie in.
+constexpr size_t kCounterBytes = (sizeof(DevCounters) + 255) & ~(size_t)255;
+
 void keep_pool_memory() {
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return;
@@ -70,11 +73,10 @@ Renderer::Renderer(std::shared_ptr<ResidentScene> scene, wf::GpuMode mode)
     cuda_check(cudaEventCreate(&ev1_), "cudaEventCreate");
     keep_pool_memory();
     // Counters and the work counter share one block from the stream-ordered pool.
-    const size_t cbytes = (sizeof(DevCounters) + 255) & ~(size_t)255;
     char* block = nullptr;
-    cuda_check(cudaMallocAsync(reinterpret_cast<void**>(&block), cbytes + 256, stream_), "allocate counters");
+    cuda_check(cudaMallocAsync(reinterpret_cast<void**>(&block), kCounterBytes + 256, stream_), "allocate counters");
     counters_ = reinterpret_cast<DevCounters*>(block);
-    work_ = reinterpret_cast<unsigned int*>(block + cbytes);
+    work_ = reinterpret_cast<unsigned int*>(block + kCounterBytes);
     alloc_film();
 }
 
@@ -123,13 +125,13 @@ void Renderer::set_camera(const wf::Camera& cam, int width, int height) {
 
 void Renderer::reset() {
     cuda_check(cudaMemsetAsync(film_.rgb, 0, 5 * (size_t)pixels() * sizeof(float), stream_), "cudaMemset film");
-    cuda_check(cudaStreamSynchronize(stream_), "cudaStreamSynchronize");
 }
 
 void Renderer::run_passes(const PassParams& p, wf::RenderStats* stats) {
     if (p.sample_count < 0 || p.first_sample < 0) throw Error(WFB_ERR_INVALID_ARGUMENT, "negative sample range");
     if (p.max_depth < 0) throw Error(WFB_ERR_INVALID_ARGUMENT, "max_depth must be >= 0");
-    cuda_check(cudaMemsetAsync(counters_, 0, sizeof(DevCounters), stream_), "zero counters");
+    // the counters and, behind them, the first launch's work counter
+    cuda_check(cudaMemsetAsync(counters_, 0, kCounterBytes + sizeof(unsigned int), stream_), "zero counters");
     // Automatic splitting: a megakernel render whose per-sample buffer would pass the cap runs as
     // consecutive sub-passes of sample ranges; each pixel still gets its samples in ascending order,
     // so the film is the same. The sample buffer is sized for the largest sub-pass before the
@@ -165,16 +167,17 @@ void Renderer::run_passes(const PassParams& p, wf::RenderStats* stats) {
             if (chunks > 1 && 3 * (size_t)pixels() * (size_t)q.sample_count > lbuf_floats_)
                 throw Error(WFB_ERR_INTERNAL, "sample buffer smaller than a sub-pass");
             last_launches_ +=
-                launch_megakernel(view_, film_, counters_, work_, lbuf_, q, mk_cfg_, chunks, stream_, &ktimer_);
+                launch_megakernel(view_, film_, counters_, work_, lbuf_, q, mk_cfg_, chunks, stream_, &ktimer_, done == 0);
         }
     } else {
         last_launches_ =
             wf_->engine.run(view_, film_, counters_, p, stats ? &stats->stages : nullptr, stream_, &ktimer_);
     }
     cuda_check(cudaEventRecord(ev1_, stream_), "cudaEventRecord");
-    cuda_check(cudaEventSynchronize(ev1_), "render");
+    // one wait for the render and its counters (a copy into pageable memory returns when it has arrived)
     DevCounters c{};
-    cuda_check(cudaMemcpy(&c, counters_, sizeof(c), cudaMemcpyDeviceToHost), "download counters");
+    cuda_check(cudaMemcpyAsync(&c, counters_, sizeof(c), cudaMemcpyDeviceToHost, stream_), "download counters");
+    cuda_check(cudaStreamSynchronize(stream_), "render");
     if (c.error != kErrNone)
         throw Error(WFB_ERR_DEVICE_WAIT, "a bounded device-side wait gave up; the render is incomplete");
     last_kernel_ms_ = ktimer_.total_ms();
@@ -202,6 +205,9 @@ void Renderer::download_sums(float* rgb_sum, float* lum_sum, float* lum2_sum) {
     if (lum2_sum) cuda_check(cudaMemcpy(lum2_sum, film_.lum2, p * sizeof(float), cudaMemcpyDeviceToHost), "download lum2");
 }
 
+// Films up to this many resolved bytes (16 a pixel) cross through the pinned staging (64x36: 41 -> 29 us, 320x180: 110 -> 87).
+constexpr size_t kStagedFilmBytes = 1u << 20;
+
 void film_download(const DevFilm& film, int spp_done, float* rgb, float* lum_var, cudaStream_t stream) {
     if (spp_done <= 0) throw Error(WFB_ERR_INVALID_ARGUMENT, "spp_done must be positive");
     if (!rgb && !lum_var) return;
@@ -213,6 +219,25 @@ void film_download(const DevFilm& film, int spp_done, float* rgb, float* lum_var
     film_resolve<<<(unsigned)((p + 255) / 256), 256, 0, s>>>(film, spp_done, rgb ? out : nullptr,
                                                               lum_var ? out + 3 * p : nullptr);
     cudaError_t e = cudaGetLastError();
+    // A small film crosses in one copy into the pinned upload staging (unless an upload is using it) and from there into the
+    // caller's buffers: two copies into pageable memory cost more than that up to about a megabyte.
+    if (4 * p * sizeof(float) <= kStagedFilmBytes) {
+        const StagingLock stage;
+        if (stage.data && stage.bytes >= 4 * p * sizeof(float)) {
+            const size_t from = rgb ? 0 : 3 * p, n = (rgb && lum_var) ? 4 * p : rgb ? 3 * p : p;
+            if (e == cudaSuccess)
+                e = cudaMemcpyAsync(stage.data, out + from, n * sizeof(float), cudaMemcpyDeviceToHost, s);
+            const cudaError_t ef = cudaFreeAsync(out, s);
+            const cudaError_t es = cudaStreamSynchronize(s);
+            cuda_check(e, "download film");
+            cuda_check(ef, "free download");
+            cuda_check(es, "cudaStreamSynchronize");
+            const float* h = reinterpret_cast<const float*>(stage.data);
+            if (rgb) std::memcpy(rgb, h, 3 * p * sizeof(float));
+            if (lum_var) std::memcpy(lum_var, h + (rgb ? 3 * p : 0), p * sizeof(float));
+            return;
+        }
+    }
     if (e == cudaSuccess && rgb) e = cudaMemcpyAsync(rgb, out, 3 * p * sizeof(float), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess && lum_var)
         e = cudaMemcpyAsync(lum_var, out + 3 * p, p * sizeof(float), cudaMemcpyDeviceToHost, s);
