@@ -83,7 +83,7 @@ void traverse_check(const wf::Scene& host, const float* rays, int n, bool anyhit
 void traverse_wide_check(const wf::Scene& host, const float* rays, int n, bool anyhit, float* hits,
                          long long* counts);
 // Host run of the ordered traversal (wide_bvh.cuh) on the host-built wide tree; counts[4]: wide nodes,
-// primitives of the leaves entered, rays handed to the preorder steps, wide nodes in the tree (0: it does not qualify,
+// primitive tests, rays handed to the preorder steps, wide nodes in the tree (0: it does not qualify,
 // and every ray takes the preorder steps).
 void traverse_ordered_check(const wf::Scene& host, const float* rays, int n, bool anyhit, float* hits,
                             long long* counts);

@@ -104,7 +104,7 @@ __global__ void __launch_bounds__(kBlock, kCtas) megakernel_wide(const WideArgs 
             const int np = __popc(pm);
             if (np != 0 && (np >= a.leaf_batch || np >= __popc(nm))) {
                 if (in_leaf) {
-                    wide_leaf_step(MULTI ? jprims : a.job0.s.prims, MULTI ? jn_spheres : a.job0.s.n_spheres, o, ray,
+                    wide_prim_step(MULTI ? jprims : a.job0.s.prims, MULTI ? jn_spheres : a.job0.s.n_spheres, o, ray,
                                    kind == kShadow, ws);
                     wide_next(ws, stack);
                 }

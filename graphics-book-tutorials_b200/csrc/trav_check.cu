@@ -266,8 +266,8 @@ void traverse_ordered_check(const wf::Scene& host, const float* rays, int n, boo
             wide_begin(d, r[7], true, 0, &ray, &s);
             while (s.cur != 0 || s.pend != 0) {
                 if (s.pend != 0) {
-                    counts[1] += s.pend & kLeafCountMask;
-                    wide_leaf_step(prims.data(), ns, o, ray, anyhit, s);
+                    ++counts[1];
+                    wide_prim_step(prims.data(), ns, o, ray, anyhit, s);
                 } else {
                     ++counts[0];
                     wide_node_step(wide.data(), o, ray.inv_d, s, stack);

@@ -309,7 +309,7 @@ __device__ void traverse_phase(const WfArgs& a, const uint32_t* items, unsigned 
             const int np = __popc(pm);
             if (np != 0 && (np >= a.leaf_batch || np >= __popc(bm))) {
                 if (in_leaf && WIDE) {
-                    wide_leaf_step(MULTI ? prims : a.job0.s.prims, MULTI ? n_spheres : a.job0.s.n_spheres, o, ray, SHADOW,
+                    wide_prim_step(MULTI ? prims : a.job0.s.prims, MULTI ? n_spheres : a.job0.s.n_spheres, o, ray, SHADOW,
                                    ws);
                     wide_next(ws, stack);
                 } else if (in_leaf) {

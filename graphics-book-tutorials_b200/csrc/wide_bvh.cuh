@@ -216,47 +216,57 @@ WF_HD void wide_node_step(const float4* __restrict__ wide, const wf::Vec3& o, co
     stack.push3(s, c1, p1, c2, p2, c3, p3);
 }
 
-// The primitives of the pending leaf against the ray, each as prim_step tests it. Closest hit: hits up to
+// The third vector of a primitive record. It is loaded along with the first two although spheres have no use for it: left to
+// the branch that uses it (where the compiler moves a plain load), it waits for the first vector to arrive.
+WF_HD float4 load_e2(const float4* rec) {
+#if defined(__CUDA_ARCH__)
+    float4 v;
+    asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                 : "l"(rec + 2));
+    return v;
+#else
+    return rec[2];
+#endif
+}
+
+// One primitive of the pending leaf against the ray, as prim_step tests it. Closest hit: hits up to
 // best * kTieUp are seen, so that a tie on either side of the best sets `redo`; a clearly nearer hit
 // clears it again. Any hit: the first hit ends the query (wide_resolve runs its leaf's own box test).
-WF_HD void wide_leaf_step(const float4* __restrict__ prims, int n_spheres, const wf::Vec3& o, const TravRay& ray,
+WF_HD void wide_prim_step(const float4* __restrict__ prims, int n_spheres, const wf::Vec3& o, const TravRay& ray,
                           bool anyhit, WideState& s) {
-    {
-        const int rank = s.pend >> kLeafCountBits;
-        const float4* rec = prims + 3 * rank;
-        const float4 q0 = ro_load(rec);
-        const float4 q1 = ro_load(rec + 1);
-        wf::Ray r;
-        r.o = o;
-        r.d = ray.d;
-        r.tmin = wf::kRayEps;
-        r.tmax = anyhit ? s.best : s.best * kTieUp;
-        float t, u, v;
-        bool hit;
-        if (f2i(q0.w) < n_spheres) {
-            hit = wf::hit_sphere_core(wf::Vec3{q0.x, q0.y, q0.z}, q1.x, r, &t);
-        } else {
-            const float4 q2 = ro_load(rec + 2);
-            hit = wf::hit_triangle_core(wf::Vec3{q0.x, q0.y, q0.z}, wf::Vec3{q1.x, q1.y, q1.z},
-                                        wf::Vec3{q2.x, q2.y, q2.z}, r, &t, &u, &v);
-        }
-        s.pend += (1 << kLeafCountBits) - 1;
-        if (hit) {
-            if (anyhit) {
-                s.rank = rank;
-                s.cur = 0;
-                s.pend = 0;
-                s.sp = s.base;
-            } else {
-                s.redo = (s.redo & ~kRedoTie) | (t >= s.best * kTieDown ? kRedoTie : 0);
-                if (t < s.best) {
-                    s.best = t;
-                    s.rank = rank;
-                }
-            }
-        }
-    }
+    const int rank = s.pend >> kLeafCountBits;
+    const float4* rec = prims + 3 * rank;
+    const float4 q2 = load_e2(rec);
+    const float4 q0 = ro_load(rec);
+    const float4 q1 = ro_load(rec + 1);
+    wf::Ray r;
+    r.o = o;
+    r.d = ray.d;
+    r.tmin = wf::kRayEps;
+    r.tmax = anyhit ? s.best : s.best * kTieUp;
+    float t, u, v;
+    bool hit;
+    if (f2i(q0.w) < n_spheres)
+        hit = wf::hit_sphere_core(wf::Vec3{q0.x, q0.y, q0.z}, q1.x, r, &t);
+    else
+        hit = wf::hit_triangle_core(wf::Vec3{q0.x, q0.y, q0.z}, wf::Vec3{q1.x, q1.y, q1.z},
+                                    wf::Vec3{q2.x, q2.y, q2.z}, r, &t, &u, &v);
+    s.pend += (1 << kLeafCountBits) - 1;
     if ((s.pend & kLeafCountMask) == 0) s.pend = 0;
+    if (!hit) return;
+    if (anyhit) {
+        s.rank = rank;
+        s.cur = 0;
+        s.pend = 0;
+        s.sp = s.base;
+        return;
+    }
+    s.redo = (s.redo & ~kRedoTie) | (t >= s.best * kTieDown ? kRedoTie : 0);
+    if (t < s.best) {
+        s.best = t;
+        s.rank = rank;
+    }
 }
 
 // The preorder steps from the ray's start: what the ordered traversal hands over to.
