@@ -243,10 +243,11 @@ struct WavefrontConfig {
     int leaf_batch = 0;       // a warp tests primitives once this many lanes hold a pending leaf; 0: the default
     bool speculate = true;    // as in MegakernelConfig
 };
-// The defaults, for the preorder steps and the ordered traversal (its rays are fetched again sooner than they would trace
-// on with few lanes, and its 64-register form is the faster one; icospheres 1280x720x16 at 10 CTAs and 24, 8 and 8, 8:
-// 19.4 / 18.7 ms, with 16 for the primitive rounds 18.5; heightfield 13.3 / 12.5 / 11.7).
-constexpr int kWfOccupancy[2] = {10, 8}, kWfMinActive[2] = {24, 8}, kWfLeafBatch[2] = {8, 16};
+// The defaults for the preorder steps, the ordered traversal, and the ordered traversal over a small tree (kSmallTree). Ordered
+// rays are fetched again sooner than they would trace on with few lanes, and its 64-register form is the faster one
+// (icospheres 1280x720x16 at 10 / 8 / 6 CTAs: 15.9 / 14.6 / 14.9 ms, heightfield 10.9 / 10.3 / 11.0); over a small tree
+// the barriers count more than the latency of the nodes (cornell36 320x180x16: 1.60 / 1.36 / 1.18 ms).
+constexpr int kWfOccupancy[3] = {10, 8, 6}, kWfMinActive[3] = {24, 8, 8}, kWfLeafBatch[3] = {8, 16, 16};
 
 // Launch configuration of a batch or a server: the arm and its knobs.
 struct LaunchConfig {

@@ -12,16 +12,15 @@
 // sample order (direct mode) or per (pixel, sample) in a buffer committed in order afterwards
 // (split mode), so the film is bit-identical to every arm.
 //
-// One bounce = five phases separated by grid barriers (bounded spins, error flag on timeout):
+// One bounce = four phases separated by grid barriers (bounded spins, error flag on timeout):
 //   R  regenerate + compact: ended slots commit their sample and start the next one (or fetch a
-//      unit, or go idle); a decoupled-look-back scan over the active list writes the next active
-//      list, stable, and its length.
+//      unit, or go idle); the slots that still have a path make the next active list, tile by tile.
 //   E  extend: closest-hit traversal of every active path, lanes fetching rays dynamically from
-//      the active list (one atomic per warp per refill) and stepping a resumable stackless
-//      traversal, so a warp never waits for its longest ray.
-//   C  classify: validity check, emission/MIS/termination; slots pushed to the Lambertian, metal or
-//      dielectric queue with warp-aggregated pushes (drop-and-count past the test capacity).
-//   S  shade: the three material queues (shade_lambert pushes shadow records).
+//      the active list (one atomic per warp per refill), so a warp never waits for its longest ray.
+//   C+S classify and shade each path where it is: validity check, emission/MIS/termination, scattering; Lambertian
+//      bounces push shadow records. Through material queues the same work took a barrier and a second read of the path
+//      state more (icospheres 1280x720x16: 4.2 -> 2.7 ms); the queues remain, as phases C and S, for stage timing
+//      and for the queue-capacity test hook (warp-aggregated pushes, drop-and-count past the capacity).
 //   H  shadow: any-hit traversal of the shadow queue with dynamic fetch; unoccluded contributions
 //      are added to the path radiance (a slot has at most one shadow record per bounce).
 // Stage times come from %globaltimer at the barriers (no host synchronisation).
@@ -53,7 +52,6 @@ struct Control {
     unsigned qcount[4];  // lambert, metal, dielectric, shadow
     unsigned fetch[2];   // extend, shadow dynamic-fetch cursors
     unsigned unit_next;
-    unsigned ticket;
     unsigned retired;    // extension rays finished in the current E phase
     unsigned suspended;  // extension rays carried over to the next iteration (all phases)
     unsigned err;
@@ -81,7 +79,6 @@ struct Pool {
     uint32_t* queue[4];  // lambert, metal, dielectric, shadow slots
     float4* sh_dir;      // shadow records: direction, tmax
     float4* sh_c;        // contribution, owner slot
-    unsigned long long* status;
     Control* ctl;
 };
 
@@ -95,6 +92,7 @@ struct WfArgs {
     int min_active;
     int leaf_batch;
     int split_shading;  // stage timing: a barrier between material queues
+    int fused;          // classify and shade in one phase, without material queues (not with stage timing or the queue test hook)
     int suspend;        // extension stragglers may be suspended to the next iteration
     int speculate;      // speculative traversal (box_step)
     unsigned long long wait_ns;  // limit of every bounded wait (grid barriers, look-backs)
@@ -366,6 +364,40 @@ __device__ void traverse_phase(const WfArgs& a, const uint32_t* items, unsigned 
     }
 }
 
+// Slots per thread and per CTA of a regeneration tile: a quarter of the atomics of one slot per thread (16M slots take 28,672
+// tiles), and no look-back chain between tiles (compact stage, icospheres 1280x720x16: 2.2 -> 1.1 ms).
+constexpr int kRegenSlots = 4;
+constexpr unsigned kRegenTile = kRegenSlots * kWfBlock;
+
+// Places for the tile's elements with `on` set: *counter grows by their number, and element (k, thread) gets the old value
+// plus the number of elements before it (k first, then thread). Every thread of the CTA calls it; `count` holds a
+// word per k and warp.
+__device__ __forceinline__ void tile_places(const bool (&on)[kRegenSlots], unsigned* counter, unsigned* count,
+                                            unsigned* base, unsigned (&at)[kRegenSlots]) {
+    constexpr int kWarps = kWfBlock / 32;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    __syncthreads();  // count and base may still be read from a previous call
+#pragma unroll
+    for (int k = 0; k < kRegenSlots; ++k) {
+        const unsigned m = __ballot_sync(kFull, on[k]);
+        at[k] = __popc(m & ((1u << lane) - 1u));
+        if (lane == 0) count[k * kWarps + warp] = __popc(m);
+    }
+    __syncthreads();
+    unsigned total = 0;
+#pragma unroll
+    for (int j = 0; j < kRegenSlots * kWarps; ++j) {
+#pragma unroll
+        for (int k = 0; k < kRegenSlots; ++k)
+            if (j == k * kWarps + warp) at[k] += total;
+        total += count[j];
+    }
+    if (threadIdx.x == 0) *base = total ? atomicAdd(counter, total) : 0u;
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kRegenSlots; ++k) at[k] += *base;
+}
+
 // MINB > 1 caps registers so that MINB CTAs fit an SM (the whole bounce loop is one kernel, so its
 // register count is the largest of any phase's; the traversal phases want the warps more than the
 // shading phases want the registers).
@@ -379,9 +411,8 @@ __global__ void __launch_bounds__(kWfBlock, MINB) wavefront_persistent(const WfA
     const int gthreads = gridDim.x * blockDim.x;
     const unsigned total_units = MULTI ? a.hdr->total_units : a.job0.units;
     const int n_jobs = MULTI ? (int)a.hdr->n_jobs : 1;
-    __shared__ uint32_t smem[33];
-    __shared__ int s_tile;
-    __shared__ uint32_t s_prefix;
+    __shared__ unsigned s_count[kRegenSlots * kWfBlock / 32];
+    __shared__ unsigned s_base;
     __shared__ int s_stack[WIDE ? kStackShared * kWfBlock : 1];
     unsigned long long t_last = 0;
     if (blockIdx.x == 0 && threadIdx.x == 0) t_last = global_ns();
@@ -400,21 +431,20 @@ __global__ void __launch_bounds__(kWfBlock, MINB) wavefront_persistent(const WfA
             c->fetch[0] = c->fetch[1] = 0;
             c->retired = 0;
         }
-        const unsigned ntiles = (n_act + kWfBlock - 1) / kWfBlock;
-        for (;;) {
-            if (threadIdx.x == 0) s_tile = (int)atomicAdd(&c->ticket, 1u);
-            __syncthreads();
-            const int tile = s_tile;
-            if (tile >= (int)ntiles) break;
-            const unsigned i = (unsigned)tile * kWfBlock + threadIdx.x;
-            const bool valid = i < n_act;
-            const int slot = valid ? (int)active[i] : 0;
-            bool has_path = false, need_unit = false;
-            int4 u = make_int4(-1, 0, 0, 0);
-            if (valid) {
-                has_path = P.alive[slot] != 0u;
-                if (!has_path) {
-                    u = P.unit[slot];
+        // A CTA takes tiles of kRegenSlots slots per thread: one atomic per tile for the new units and one for the place of
+        // its slots in the next list (ordered within the tile, tiles in the order they get there).
+        for (unsigned base = (unsigned)blockIdx.x * kRegenTile; base < n_act; base += gridDim.x * kRegenTile) {
+            int slots[kRegenSlots];
+            bool has_path[kRegenSlots], need_unit[kRegenSlots];
+#pragma unroll
+            for (int k = 0; k < kRegenSlots; ++k) {
+                const unsigned i = base + k * kWfBlock + threadIdx.x;
+                const bool valid = i < n_act;
+                const int slot = slots[k] = valid ? (int)active[i] : 0;
+                has_path[k] = valid && P.alive[slot] != 0u;
+                need_unit[k] = valid && !has_path[k];
+                if (need_unit[k]) {
+                    int4 u = P.unit[slot];
                     if (u.x >= 0) {
                         const JobDesc& J = job_at<MULTI>(a, u.w);
                         const bool split = J.chunks > 1;
@@ -443,7 +473,8 @@ __global__ void __launch_bounds__(kWfBlock, MINB) wavefront_persistent(const WfA
                             store_path(P, slot, wf::init_path(J.s, px, py, (uint32_t)u.y, J.seed));
                             P.unit[slot] = u;
                             P.alive[slot] = 1u;
-                            has_path = true;
+                            has_path[k] = true;
+                            need_unit[k] = false;
                         } else {
                             if (!split) {
                                 const float4 ac = P.acc[slot];
@@ -455,68 +486,45 @@ __global__ void __launch_bounds__(kWfBlock, MINB) wavefront_persistent(const WfA
                             }
                             u.x = -1;
                             P.unit[slot] = u;
-                            need_unit = true;
                         }
-                    } else {
-                        need_unit = true;
                     }
                 }
             }
-            // fetch new units for slots that need one (one atomic per warp)
-            const unsigned nm = __ballot_sync(kFull, need_unit);
-            if (nm) {
-                const int leader = __ffs(nm) - 1;
-                unsigned base = 0;
-                if (lane == leader) base = atomicAdd(&c->unit_next, (unsigned)__popc(nm));
-                base = __shfl_sync(kFull, base, leader);
-                if (need_unit) {
-                    const unsigned uid = base + __popc(nm & ((1u << lane) - 1u));
-                    if (uid < total_units) {
-                        // unit -> job, then pixel (local mod P) and chunk (local div P)
-                        const int job = MULTI ? job_of_unit(a.jobs, n_jobs, uid) : 0;
-                        const JobDesc& J = job_at<MULTI>(a, job);
-                        const unsigned local = uid - J.unit_begin;
-                        const int pixel = (int)(local % (unsigned)J.film.pixels);
-                        const int ch = (int)(local / (unsigned)J.film.pixels);
-                        const int first = J.first_sample + ch * J.chunk;
-                        const int end = min(first + J.chunk, J.first_sample + J.sample_count);
-                        P.unit[slot] = make_int4(pixel, first, end, job);
-                        if (J.chunks == 1) {
-                            P.acc[slot] = make_float4(J.film.rgb[3 * pixel], J.film.rgb[3 * pixel + 1],
-                                                      J.film.rgb[3 * pixel + 2], J.film.lum[pixel]);
-                            P.acc2[slot] = J.film.lum2[pixel];
-                        }
-                        store_path(P, slot, wf::init_path(J.s, pixel % J.s.width, pixel / J.s.width, (uint32_t)first, J.seed));
-                        P.alive[slot] = 1u;
-                        has_path = true;
+            unsigned at[kRegenSlots];
+            tile_places(need_unit, &c->unit_next, s_count, &s_base, at);
+#pragma unroll
+            for (int k = 0; k < kRegenSlots; ++k) {
+                const unsigned uid = at[k];
+                if (need_unit[k] && uid < total_units) {
+                    // unit -> job, then pixel (local mod P) and chunk (local div P)
+                    const int slot = slots[k];
+                    const int job = MULTI ? job_of_unit(a.jobs, n_jobs, uid) : 0;
+                    const JobDesc& J = job_at<MULTI>(a, job);
+                    const unsigned local = uid - J.unit_begin;
+                    const int pixel = (int)(local % (unsigned)J.film.pixels);
+                    const int ch = (int)(local / (unsigned)J.film.pixels);
+                    const int first = J.first_sample + ch * J.chunk;
+                    const int end = min(first + J.chunk, J.first_sample + J.sample_count);
+                    P.unit[slot] = make_int4(pixel, first, end, job);
+                    if (J.chunks == 1) {
+                        P.acc[slot] = make_float4(J.film.rgb[3 * pixel], J.film.rgb[3 * pixel + 1],
+                                                  J.film.rgb[3 * pixel + 2], J.film.lum[pixel]);
+                        P.acc2[slot] = J.film.lum2[pixel];
                     }
+                    store_path(P, slot, wf::init_path(J.s, pixel % J.s.width, pixel / J.s.width, (uint32_t)first, J.seed));
+                    P.alive[slot] = 1u;
+                    has_path[k] = true;
                 }
             }
-            // stable compaction of the slots that still have a path
-            const uint32_t flag = (valid && has_path) ? 1u : 0u;
-            uint32_t agg;
-            const uint32_t excl = block_exclusive_sum(flag, smem, &agg);
-            if (threadIdx.x == 0) publish_status(P.status, tile, iter, tile == 0 ? kStatusPrefix : kStatusAggregate, agg);
-            if (tile > 0 && threadIdx.x < 32) {
-                const uint32_t pre = tile_lookback(P.status, tile, iter, &c->err, a.wait_ns);
-                if (threadIdx.x == 0) {
-                    publish_status(P.status, tile, iter, kStatusPrefix, pre + agg);
-                    s_prefix = pre;
-                }
-            } else if (tile == 0 && threadIdx.x == 0) {
-                s_prefix = 0;
-            }
-            __syncthreads();
-            if (flag) next[s_prefix + excl] = (uint32_t)slot;
-            if (tile == (int)ntiles - 1 && threadIdx.x == kWfBlock - 1) c->n_next = s_prefix + excl + flag;
-            __syncthreads();
+            tile_places(has_path, &c->n_next, s_count, &s_base, at);
+#pragma unroll
+            for (int k = 0; k < kRegenSlots; ++k)
+                if (has_path[k]) next[at[k]] = (uint32_t)slots[k];
         }
-        if (ntiles == 0 && gtid == 0) c->n_next = 0;
         if (!grid_sync(c, nblocks, 6, &t_last, a.wait_ns)) break;
         const unsigned n = *(volatile unsigned*)&c->n_next;
         if (gtid == 0) {
             c->n_active = n;
-            c->ticket = 0;
             if (n > c->high_water[4]) c->high_water[4] = n;
         }
         if (n == 0) break;
@@ -526,7 +534,57 @@ __global__ void __launch_bounds__(kWfBlock, MINB) wavefront_persistent(const WfA
         traverse_phase<false, MULTI, WIDE>(a, next, n, &c->fetch[0], &n_ext, s_stack, &c->retired,
                                      a.suspend && n >= 4096 ? n - n / 20 : 0xffffffffu);
         if (!grid_sync(c, nblocks, 0, &t_last, a.wait_ns)) break;
+        if (gtid == 0) c->n_next = 0;  // every CTA has read it; the next regeneration counts from 0
 
+        if (a.fused) {
+            // ---------------- C + S in one: classify and shade each path where it is ----------------
+            unsigned count[3] = {0, 0, 0};  // per warp, as its material queues would have had them
+            for (unsigned base = (unsigned)blockIdx.x * kWfBlock; base < n; base += (unsigned)gthreads) {
+                const unsigned i = base + threadIdx.x;
+                const int slot = i < n ? (int)next[i] : 0;
+                int mat = -1, has = 0;
+                wf::Ray sh;
+                wf::Vec3 contrib{0.f, 0.f, 0.f};
+                if (i < n && P.alive[slot] != 2u) {  // a suspended ray has no hit yet
+                    const float4 hv = P.hit[slot];
+                    wf::HitRecord h;
+                    h.t = hv.x;
+                    h.prim = __float_as_int(hv.y);
+                    h.u = hv.z;
+                    h.v = hv.w;
+                    const JobDesc& J = job_at<MULTI>(a, MULTI ? P.unit[slot].w : 0);
+                    if (!hit_is_valid(J.s, h)) {
+                        ++n_invalid;
+                        h.prim = -1;  // treated as a miss
+                    }
+                    wf::PathState ps = load_path(P, slot);
+                    wf::Surface f;
+                    wf::Material m;
+                    mat = wf::classify(J.s, ps, h, J.max_depth, &f, &m);
+                    if (mat < 0) {
+                        store_radiance(P, slot, ps);
+                        P.alive[slot] = 0u;
+                    } else {
+                        const bool alive = wf::shade(J.s, ps, f, m, mat, &sh, &contrib, &has);
+                        store_path(P, slot, ps);
+                        P.alive[slot] = alive ? 1u : 0u;
+                    }
+                }
+#pragma unroll
+                for (int q = 0; q < 3; ++q) count[q] += __popc(__ballot_sync(kFull, mat == q));
+                const uint32_t at = queue_push(P.queue[3], &c->qcount[3], a.qcap, (uint32_t)slot, has != 0, &c->overflow);
+                if (has && at != 0xFFFFFFFFu) {
+                    P.sh_dir[at] = make_float4(sh.d.x, sh.d.y, sh.d.z, sh.tmax);
+                    P.sh_c[at] = make_float4(contrib.x, contrib.y, contrib.z, __int_as_float(slot));
+                }
+            }
+            if (lane == 0)
+                for (int q = 0; q < 3; ++q)
+                    if (count[q]) atomicAdd(&c->qcount[q], count[q]);
+            if (!grid_sync(c, nblocks, 1, &t_last, a.wait_ns)) break;
+            if (gtid == 0)
+                for (int q = 0; q < 3; ++q) c->high_water[q] = max(c->high_water[q], *(volatile unsigned*)&c->qcount[q]);
+        } else {
         // ---------------- C: classify, push material queues ----------------
         for (unsigned base = (unsigned)blockIdx.x * kWfBlock; base < n; base += (unsigned)gthreads) {
             const unsigned i = base + threadIdx.x;
@@ -611,6 +669,7 @@ __global__ void __launch_bounds__(kWfBlock, MINB) wavefront_persistent(const WfA
         }
         if (!ok) break;
         if (!a.split_shading && !grid_sync(c, nblocks, 2, &t_last, a.wait_ns)) break;
+        }
 
         // ---------------- H: shadow rays ----------------
         const unsigned nsh = min(*(volatile unsigned*)&c->qcount[3], a.qcap);
@@ -645,13 +704,15 @@ WfKernel wavefront_kernel(int occupancy) {
     }
 }
 
-__global__ void wavefront_init(Pool P, int capacity) {
+// No more slots than the launch has units start out active.
+__global__ void wavefront_init(Pool P, int capacity, unsigned units, const BatchHeader* hdr) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int n = (int)min((unsigned)capacity, hdr ? hdr->total_units : units);
     if (i == 0) {
         Control* c = P.ctl;
-        c->n_active = (unsigned)capacity;
+        c->n_active = (unsigned)n;
     }
-    if (i < capacity) {
+    if (i < n) {
         P.list[0][i] = (uint32_t)i;
         P.alive[i] = 0u;
         P.unit[i] = make_int4(-1, 0, 0, 0);
@@ -696,7 +757,6 @@ size_t pool_bytes(int cap, Pool* out, char* base) {
     for (int q = 0; q < 4; ++q) P.queue[q] = carve<uint32_t>(p, cap);
     P.sh_dir = carve<float4>(p, cap);
     P.sh_c = carve<float4>(p, cap);
-    P.status = carve<unsigned long long>(p, (size_t)cap / kWfBlock + 2);
     P.ctl = carve<Control>(p, 1);
     if (out) *out = P;
     return (size_t)(p - base);
@@ -709,10 +769,10 @@ struct WavefrontEngine::State {
     float* lbuf = nullptr;
     size_t lbuf_floats = 0;
     void* acc = nullptr;  // direct-mode film sums per slot (float4 + float), allocated on first use
-    // the register-cap variants of cfg.occupancy and their co-resident CTAs: [0] preorder, [1] ordered traversal; for
-    // single renders and for batches
-    WfKernel kernel[2] = {}, kernel_multi[2] = {};
-    int grid[2] = {}, grid_multi[2] = {};
+    // the register-cap variants of cfg.occupancy and their co-resident CTAs: [0] preorder, [1] ordered traversal, [2]
+    // ordered over a small tree; for single renders and for batches
+    WfKernel kernel[3] = {}, kernel_multi[3] = {};
+    int grid[3] = {}, grid_multi[3] = {};
     // L2 residency: an access-policy window over the pool arena on every launch (0 bytes: none)
     size_t window_bytes = 0;
     float hit_ratio = 0.f;
@@ -785,13 +845,10 @@ WavefrontEngine::WavefrontEngine(int pixels, const WavefrontConfig& cfg) : pixel
     cuda_check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "SM count");
     if (cfg.occupancy > 0 && cfg.occupancy != 6 && cfg.occupancy != 8 && cfg.occupancy != 10)
         throw Error(WFB_ERR_INVALID_ARGUMENT, "wavefront occupancy target must be 0, 6, 8 or 10");
-    const int cap_preorder = cfg.occupancy >= 0 ? cfg.occupancy : kWfOccupancy[0];
-    const int cap_ordered = cfg.occupancy >= 0 ? cfg.occupancy : kWfOccupancy[1];
-    state_->kernel[0] = wavefront_kernel<false, false>(cap_preorder);
-    state_->kernel[1] = wavefront_kernel<false, true>(cap_ordered);
-    state_->kernel_multi[0] = wavefront_kernel<true, false>(cap_preorder);
-    state_->kernel_multi[1] = wavefront_kernel<true, true>(cap_ordered);
-    for (int w = 0; w < 2; ++w) {
+    for (int w = 0; w < 3; ++w) {
+        const int cap_ctas = cfg.occupancy >= 0 ? cfg.occupancy : kWfOccupancy[w];
+        state_->kernel[w] = w ? wavefront_kernel<false, true>(cap_ctas) : wavefront_kernel<false, false>(cap_ctas);
+        state_->kernel_multi[w] = w ? wavefront_kernel<true, true>(cap_ctas) : wavefront_kernel<true, false>(cap_ctas);
         cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, state_->kernel[w], kWfBlock, 0), "occupancy");
         if (occ < 1) throw Error(WFB_ERR_UNSUPPORTED, "wavefront kernel does not fit on an SM");
         state_->grid[w] = sms * occ;
@@ -845,9 +902,7 @@ int launch_pool(WfKernel kernel, const WfArgs& args, int grid, int capacity, Dev
                 size_t window_bytes, float hit_ratio, cudaStream_t stream, KernelTimer* timer = nullptr) {
     const Pool& pool = args.pool;
     cuda_check(cudaMemsetAsync(pool.ctl, 0, sizeof(Control), stream), "memset control");
-    cuda_check(cudaMemsetAsync(pool.status, 0, ((size_t)capacity / kWfBlock + 2) * sizeof(unsigned long long), stream),
-               "memset status");
-    wavefront_init<<<(capacity + 255) / 256, 256, 0, stream>>>(pool, capacity);
+    wavefront_init<<<(capacity + 255) / 256, 256, 0, stream>>>(pool, capacity, args.job0.units, args.hdr);
     cuda_check(cudaGetLastError(), "wavefront init launch");
     WfArgs a = args;
     a.wait_ns = device_wait_limit_ns();
@@ -909,7 +964,7 @@ int WavefrontEngine::run(const DevScene& s, const DevFilm& film, DevCounters* co
                          wf::StageTimes* stages, cudaStream_t stream, KernelTimer* timer) {
     if (p.sample_count <= 0 || film.pixels <= 0) return 0;
     State& st = *state_;
-    const int w = cfg_.speculate && wide_usable(s) ? 1 : 0;
+    const int w = !cfg_.speculate || !wide_usable(s) ? 0 : s.n_nodes < kSmallTree ? 2 : 1;
     const int chunks = chunks_for(film.pixels, p.sample_count);
     WfArgs a{};
     a.job0 = make_job(s, film, nullptr, p.first_sample, p.sample_count, chunks, p.seed, p.max_depth);
@@ -927,6 +982,7 @@ int WavefrontEngine::run(const DevScene& s, const DevFilm& film, DevCounters* co
     a.min_active = cfg_.min_active > 0 ? cfg_.min_active : kWfMinActive[w];
     a.leaf_batch = cfg_.leaf_batch > 0 ? cfg_.leaf_batch : kWfLeafBatch[w];
     a.split_shading = p.stage_timing ? 1 : 0;
+    a.fused = !p.stage_timing && a.qcap >= (uint32_t)capacity_ ? 1 : 0;
     a.suspend = cfg_.suspend_stragglers ? 1 : 0;
     a.speculate = cfg_.speculate ? 1 : 0;
     int launches = launch_pool(st.kernel[w], a, st.grid[w], capacity_, counters, p.count_rays, st.window_bytes, st.hit_ratio,
@@ -952,9 +1008,9 @@ int WavefrontEngine::run(const DevScene& s, const DevFilm& film, DevCounters* co
 }
 
 int WavefrontEngine::run_batch(const JobDesc* d_jobs, const BatchHeader* d_hdr, DevCounters* counters,
-                               bool count_rays, bool all_wide, cudaStream_t stream) {
+                               bool count_rays, int wide_nodes, cudaStream_t stream) {
     reserve_direct();  // a batch may hold direct-mode jobs
-    const int w = cfg_.speculate && all_wide ? 1 : 0;
+    const int w = !cfg_.speculate || wide_nodes == 0 ? 0 : wide_nodes < kSmallTree ? 2 : 1;
     WfArgs a{};
     a.jobs = d_jobs;
     a.hdr = d_hdr;
@@ -964,6 +1020,7 @@ int WavefrontEngine::run_batch(const JobDesc* d_jobs, const BatchHeader* d_hdr, 
     a.min_active = cfg_.min_active > 0 ? cfg_.min_active : kWfMinActive[w];
     a.leaf_batch = cfg_.leaf_batch > 0 ? cfg_.leaf_batch : kWfLeafBatch[w];
     a.split_shading = 0;
+    a.fused = 1;
     a.suspend = cfg_.suspend_stragglers ? 1 : 0;
     a.speculate = cfg_.speculate ? 1 : 0;
     return launch_pool(state_->kernel_multi[w], a, state_->grid_multi[w], capacity_, counters, count_rays, state_->window_bytes,

@@ -25,7 +25,7 @@ public:
     // megakernel) in one cooperative launch; the caller commits split-mode films afterwards
     // (launch_film_commit_jobs). Returns the number of kernels launched.
     int run_batch(const JobDesc* d_jobs, const BatchHeader* d_hdr, DevCounters* counters, bool count_rays,
-                  bool all_wide, cudaStream_t stream);
+                  int wide_nodes, cudaStream_t stream);
     uint64_t bytes() const;
     int capacity() const { return capacity_; }
     // Bytes of the pool under a persisting L2 access-policy window on every launch (0: none).
