@@ -106,6 +106,54 @@ def test_trees_that_do_not_qualify(wfb, orc, how):
     assert _same(got, orc.intersect(arrays, rays))
 
 
+def _chain(wfb, n, overlap):
+    """A BVH that is a chain: every internal node has one leaf and the rest. Triangles in a row along x; with `overlap`
+    stacked along z instead, so that a ray along z meets every box."""
+    rng = np.random.default_rng(n)
+    base = wfb.Scene.generate("cornell36", 24, 16, 1234, 16).export()
+    verts = np.zeros((3 * n, 3), np.float32)
+    for k in range(n):
+        at = np.array([0.5, 0.5, -0.01 * k] if overlap else [k / n, 0.5, 0.0])
+        verts[3 * k : 3 * k + 3] = at + rng.uniform(-0.4, 0.4, (3, 3)) * ([1, 1, 0.001] if overlap else [1 / n, 1, 0.2])
+    tris = np.zeros(n, wfb.TRIANGLE)
+    tris["i0"], tris["i1"], tris["i2"] = np.arange(n) * 3, np.arange(n) * 3 + 1, np.arange(n) * 3 + 2
+    lo, hi = verts.reshape(n, 3, 3).min(1), verts.reshape(n, 3, 3).max(1)
+    nodes = np.zeros(2 * n - 1, wfb.BVH_NODE)
+    nodes["prim_start"] = -1
+    for k in range(n):
+        leaf = 2 * k + 1 if k < n - 1 else 2 * k
+        nodes["lo"][leaf], nodes["hi"][leaf] = lo[k], hi[k]
+        nodes["prim_start"][leaf], nodes["prim_count"][leaf] = k, 1
+        nodes["skip"][leaf] = leaf + 1 if k < n - 1 else -1
+        if k < n - 1:
+            nodes["lo"][2 * k], nodes["hi"][2 * k], nodes["skip"][2 * k] = lo[k:].min(0), hi[k:].max(0), -1
+    return dict(base, vertices=verts, triangles=tris, spheres=np.zeros(0, wfb.SPHERE), nodes=nodes,
+                prim_order=np.arange(n, dtype=np.int32), lights=np.zeros(0, wfb.LIGHT), env=[1.0, 0.9, 0.8])
+
+
+# 2 triangles; one node and its levels in one block; several launches of levels and a lane stack that overflows
+# (every box met, 3 leaves left behind per level); more levels than the wide tree may have
+CHAINS = [(2, False), (100, True), (250, False), (250, True), (400, True)]
+
+
+@pytest.mark.parametrize("n,overlap", CHAINS)
+@pytest.mark.parametrize("anyhit", [False, True])
+def test_ordered_traversal_on_chains(wfb, orc, n, overlap, anyhit):
+    arrays = _chain(wfb, n, overlap)
+    scene = wfb.Scene.from_arrays(arrays)
+    rng = np.random.default_rng(5)
+    rays = _rays(wfb, arrays, 1200, seed=n)
+    rays["o"][600:] = rng.uniform([0.2, 0.2, 1.0], [0.8, 0.8, 2.0], (600, 3))  # along the stack, all boxes in a row
+    rays["d"][600:] = np.array([0.01, 0.02, -0.9997], np.float32)
+    rays["o"][900:, 2] -= np.float32(0.01 * n + 4.0)
+    rays["d"][900:, 2] = np.float32(0.9997)
+    want = orc.intersect(arrays, rays, anyhit=anyhit)
+    got, _ = scene.test_traverse_ordered(rays, anyhit=anyhit)
+    assert np.array_equal(got["prim"] >= 0, want["prim"] >= 0)
+    if not anyhit:
+        assert _same(got, want)
+
+
 def _film(wfb, scene, mode, on, spp, depth, **knobs):
     r = wfb.GpuRenderer(scene, mode)
     if knobs:
@@ -116,6 +164,30 @@ def _film(wfb, scene, mode, on, spp, depth, **knobs):
     sums = r.download_sums()
     r.close()
     return np.concatenate([s.ravel() for s in sums]).view(np.uint32)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,overlap", CHAINS)
+def test_films_of_chains(wfb, n, overlap):
+    arrays = _chain(wfb, n, overlap)
+    scene = wfb.Scene.from_arrays(arrays)
+    for mode in (wfb.MEGAKERNEL, wfb.WAVEFRONT):
+        assert np.array_equal(_film(wfb, scene, mode, True, 3, 8), _film(wfb, scene, mode, False, 3, 8))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("w,h", [(256, 255), (256, 256), (256, 257)])
+def test_downloads_either_side_of_the_staged_size(wfb, w, h):
+    """Films below, at and above 1 MB of resolved bytes, whole and in parts, against the raw sums."""
+    scene = wfb.Scene.generate("cornell36", w, h, 1234, 16)
+    r = wfb.GpuRenderer(scene, wfb.MEGAKERNEL)
+    out = r.render(wfb.RenderParams(spp=4, seed=2, max_depth=4))
+    rgb, lum, lum2 = r.download_sums()
+    inv = np.float32(1.0) / np.float32(4)
+    assert np.array_equal(out.rgb.view(np.uint32), (rgb * inv).view(np.uint32))
+    m, m2 = lum.astype(np.float64) / 4, lum2.astype(np.float64) / 4
+    assert np.array_equal(out.lum_var, np.maximum(0.0, m2 - m * m).astype(np.float32))
+    assert np.array_equal(r.download_mean(4).view(np.uint32), out.rgb.view(np.uint32))
 
 
 @pytest.mark.gpu
