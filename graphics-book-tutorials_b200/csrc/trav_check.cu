@@ -203,18 +203,18 @@ std::vector<float4> host_wide(const std::vector<float4>& nodes, int nn, std::vec
     std::vector<int> roots{0};
     std::vector<float4> wide;
     for (size_t w = 0; w < roots.size(); ++w) {
-        int kids[kWideArity], codes[kWideArity];
-        const int k = wide_children(nodes.data(), nn, roots[w], kids);
-        if (k < 0) return {};
-        for (int j = 0; j < k; ++j) {
-            codes[j] = f2i(nodes[2 * (size_t)kids[j] + 1].w);
+        WideKids kids;
+        if (!wide_children(nodes.data(), nn, roots[w], &kids)) return {};
+        int codes[kWideArity];
+        for (int j = 0; j < kWideArity; ++j) {
+            codes[j] = j < kids.n ? f2i(nodes[2 * (size_t)kids.id[j] + 1].w) : 0;
             if (codes[j] < 0) {
                 codes[j] = ~(int)roots.size();
-                roots.push_back(kids[j]);
+                roots.push_back(kids.id[j]);
             }
         }
         wide.resize((size_t)kWideFloat4 * (w + 1));
-        wide_write(nodes.data(), kids, codes, k, &wide[(size_t)kWideFloat4 * w]);
+        wide_write(nodes.data(), kids, codes, &wide[(size_t)kWideFloat4 * w]);
     }
     return wide;
 }

@@ -2,9 +2,8 @@
 // tags their primitives. Then the tree is collapsed level by level, one thread per wide node: a level's nodes are
 // numbered after all earlier levels (per-level counts), and each thread hands a child its preorder node in the
 // child's own record, so a level needs nothing but the counts of the levels before it. The first levels, up to
-// kTopNodes nodes each, run in one block of one launch (a small scene's whole tree: 2 launches instead of 17);
-// each later level is a launch of its own. A level costs the latency of its threads' walk over the preorder nodes, about
-// 10 us for a small one. Icospheres (163K leaves, 80K wide nodes): 0.14 ms in all.
+// kTopNodes nodes each, run in one block of one launch; each later level is a launch of its own; a small scene's tree
+// takes one launch in all. A level costs the latency of its threads' walk over the preorder nodes.
 #include <algorithm>
 #include <cmath>
 #include "engine.hpp"
@@ -20,16 +19,9 @@ struct WideCtl {
     int count[kWideMaxLevels + 2];  // wide nodes per level
 };
 
-// Leaves: box in range, primitives inside it, each primitive record in one leaf; tags the record with the
-// leaf's node id + 1 (the w of its second float4, 0 at upload). Thread 0 starts the tree.
-__global__ void wide_check_leaves(const float4* __restrict__ nodes, int nn, float4* prims, int n_spheres,
-                                  float4* wide, WideCtl* ctl) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i == 0) {
-        ctl->count[0] = 1;
-        reinterpret_cast<int*>(wide)[0] = 0;
-    }
-    if (i >= nn) return;
+// Node i's conditions: box in range and, for a leaf, primitives inside it, each primitive record in one leaf; tags the record
+// with the leaf's node id + 1 (the w of its second float4, 0 at upload).
+__device__ bool check_leaf(const float4* nodes, int i, float4* prims, int n_spheres) {
     const float4 lo = nodes[2 * i], hi = nodes[2 * i + 1];
     const int leaf = f2i(hi.w);
     bool ok = box_in_range(lo, hi);
@@ -42,7 +34,18 @@ __global__ void wide_check_leaves(const float4* __restrict__ nodes, int nn, floa
         }
         ok = ok && n > 0;
     }
-    if (!ok) ctl->bad = 1;
+    return ok;
+}
+
+// Checks every node; thread 0 starts the tree.
+__global__ void wide_check_leaves(const float4* __restrict__ nodes, int nn, float4* prims, int n_spheres,
+                                  float4* wide, WideCtl* ctl) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i == 0) {
+        ctl->count[0] = 1;
+        reinterpret_cast<int*>(wide)[0] = 0;
+    }
+    if (i < nn && !check_leaf(nodes, i, prims, n_spheres)) ctl->bad = 1;
 }
 
 constexpr int kTopNodes = 128;
@@ -52,39 +55,39 @@ __device__ void build_node(const float4* __restrict__ nodes, int nn, float4* wid
                            int* next_count, WideCtl* ctl) {
     float4* rec = wide + (size_t)kWideFloat4 * at;
     const int root = *reinterpret_cast<volatile int*>(rec);
-    int kids[kWideArity], codes[kWideArity], inner = 0;
-    int k = wide_children(nodes, nn, root, kids);
-    if (k < 0) {
+    WideKids kids;
+    if (!wide_children(nodes, nn, root, &kids)) {
         ctl->bad = 1;
-        k = 0;
+        return;
     }
-    for (int j = 0; j < k; ++j) {
-        codes[j] = f2i(nodes[2 * kids[j] + 1].w);
+    int codes[kWideArity], inner = 0;
+#pragma unroll
+    for (int j = 0; j < kWideArity; ++j) {
+        codes[j] = j < kids.n ? f2i(nodes[2 * kids.id[j] + 1].w) : 0;
         inner += codes[j] < 0;
     }
-    if (inner) {
-        int id = next + atomicAdd(next_count, inner);
-        for (int j = 0; j < k; ++j) {
-            if (codes[j] >= 0) continue;
-            if (id >= capacity) {
-                ctl->bad = 1;
-                codes[j] = 0;
-                continue;
-            }
-            codes[j] = ~id;
-            reinterpret_cast<int*>(wide + (size_t)kWideFloat4 * id)[0] = kids[j];
-            ++id;
+    int id = inner ? next + atomicAdd(next_count, inner) : 0;
+#pragma unroll
+    for (int j = 0; j < kWideArity; ++j) {
+        if (codes[j] >= 0) continue;
+        if (id >= capacity) {
+            ctl->bad = 1;
+            return;
         }
+        codes[j] = ~id;
+        reinterpret_cast<int*>(wide + (size_t)kWideFloat4 * id)[0] = kids.id[j];
+        ++id;
     }
-    wide_write(nodes, kids, codes, k, rec);
+    wide_write(nodes, kids, codes, rec);
 }
 
-__global__ void wide_build_top(const float4* __restrict__ nodes, int nn, float4* wide, int capacity, WideCtl* ctl) {
+// One block: levels from the first on while they hold at most `most` nodes.
+__device__ void build_levels(const float4* __restrict__ nodes, int nn, float4* wide, int capacity, int most, WideCtl* ctl) {
     volatile int* count = ctl->count;
     int begin = 0, level = 0;
     for (; level < kWideMaxLevels; ++level) {
         const int n = count[level];
-        if (n == 0 || n > kTopNodes) break;
+        if (n == 0 || n > most) break;
         for (int i = threadIdx.x; i < n && begin + i < capacity; i += blockDim.x)
             build_node(nodes, nn, wide, capacity, begin + i, begin + n, &ctl->count[level + 1], ctl);
         __threadfence();
@@ -92,6 +95,27 @@ __global__ void wide_build_top(const float4* __restrict__ nodes, int nn, float4*
         begin += n;
     }
     if (threadIdx.x == 0) ctl->top = level;
+}
+
+__global__ void wide_build_top(const float4* __restrict__ nodes, int nn, float4* wide, int capacity, WideCtl* ctl) {
+    build_levels(nodes, nn, wide, capacity, kTopNodes, ctl);
+}
+
+// A whole tree of at most kSmallNodes preorder nodes in one block, its nodes in shared memory: leaf check and levels.
+constexpr int kSmallNodes = 1024;
+__global__ void wide_build_small(const float4* __restrict__ global_nodes, int nn, float4* prims, int n_spheres,
+                                 float4* wide, int capacity, WideCtl* ctl) {
+    extern __shared__ float4 nodes[];
+    for (int i = threadIdx.x; i < 2 * nn; i += blockDim.x) nodes[i] = global_nodes[i];
+    if (threadIdx.x == 0) {
+        ctl->count[0] = 1;
+        reinterpret_cast<int*>(wide)[0] = 0;
+    }
+    __threadfence();
+    __syncthreads();
+    for (int i = threadIdx.x; i < nn; i += blockDim.x)
+        if (!check_leaf(nodes, i, prims, n_spheres)) ctl->bad = 1;
+    build_levels(nodes, nn, wide, capacity, capacity, ctl);
 }
 
 // Level `after_top` of those that wide_build_top left.
@@ -116,10 +140,15 @@ int launch_wide_build(const DevScene& s, float4* prims, float4* wide, int capaci
     (void)cudaGetLastError();  // the check below is for these launches only
     if (first_level == 0) {
         cuda_check(cudaMemsetAsync(ctl, 0, sizeof(WideCtl), stream), "memset wide build");
+        if (s.n_nodes <= kSmallNodes) {
+            wide_build_small<<<1, 256, (size_t)s.n_nodes * 32, stream>>>(s.nodes, s.n_nodes, prims, s.n_spheres, wide,
+                                                                         capacity, ctl);
+            cuda_check(cudaGetLastError(), "wide build launch");
+            return 0;
+        }
         wide_check_leaves<<<(s.n_nodes + 255) / 256, 256, 0, stream>>>(s.nodes, s.n_nodes, prims, s.n_spheres, wide, ctl);
         wide_build_top<<<1, 512, 0, stream>>>(s.nodes, s.n_nodes, wide, capacity, ctl);
-        if (capacity <= kTopNodes) levels = 0;  // no level is larger than the tree
-        else if (levels <= 0) levels = std::max(1, (int)std::ceil(0.62 * std::log2((double)capacity)) - 2);
+        if (levels <= 0) levels = std::max(1, (int)std::ceil(0.62 * std::log2((double)capacity)) - 2);
     }
     if (first_level > 0 && levels <= 0) levels = 8;
     const int grid = std::min((capacity + 63) / 64, 148 * 16);
