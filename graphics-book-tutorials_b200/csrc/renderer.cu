@@ -1,5 +1,6 @@
 // GPU renderer: one resident scene, one camera, one film (the wf::GpuRenderer contract,
 // WVM/src/gpu/gpu_renderer.cu:100-377) on this engine's kernels.
+#include <sys/mman.h>
 #include <algorithm>
 #include <cstring>
 #include <vector>
@@ -205,6 +206,22 @@ void Renderer::download_sums(float* rgb_sum, float* lum_sum, float* lum2_sum) {
     if (lum2_sum) cuda_check(cudaMemcpy(lum2_sum, film_.lum2, p * sizeof(float), cudaMemcpyDeviceToHost), "download lum2");
 }
 
+// Makes the pages of a destination that a copy is about to fill present in one call instead of a fault per page (a large film
+// usually lands in fresh memory). Pages that are present stay as they are; where the kernel has no such call, the copy's
+// own faults do the work. 16 films of 72 MB in all into fresh memory: 46 to 88 ms to download without, 22 with; into
+// memory in use before, the same 6 to 9. (On 4 threads it takes as long.)
+void populate_pages(void* p, size_t bytes) {
+#if defined(MADV_POPULATE_WRITE)
+    constexpr uintptr_t kPage = 4096;
+    const uintptr_t lo = (reinterpret_cast<uintptr_t>(p) + kPage - 1) & ~(kPage - 1);
+    const uintptr_t hi = (reinterpret_cast<uintptr_t>(p) + bytes) & ~(kPage - 1);
+    if (hi > lo) (void)madvise(reinterpret_cast<void*>(lo), hi - lo, MADV_POPULATE_WRITE);
+#else
+    (void)p;
+    (void)bytes;
+#endif
+}
+
 // Films up to this many resolved bytes (16 a pixel) cross through the pinned staging (64x36: 41 -> 29 us, 320x180: 110 -> 87).
 constexpr size_t kStagedFilmBytes = 1u << 20;
 
@@ -238,6 +255,8 @@ void film_download(const DevFilm& film, int spp_done, float* rgb, float* lum_var
             return;
         }
     }
+    if (rgb) populate_pages(rgb, 3 * p * sizeof(float));
+    if (lum_var) populate_pages(lum_var, p * sizeof(float));
     if (e == cudaSuccess && rgb) e = cudaMemcpyAsync(rgb, out, 3 * p * sizeof(float), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess && lum_var)
         e = cudaMemcpyAsync(lum_var, out + 3 * p, p * sizeof(float), cudaMemcpyDeviceToHost, s);
