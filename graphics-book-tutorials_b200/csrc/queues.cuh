@@ -2,7 +2,7 @@
 //
 //   queue_push       warp-aggregated reservation: one atomic per warp per push, drop-and-count past
 //                    the capacity (semantics of WVM/src/gpu/queues.cuh:12-27).
-//   block_scan       exclusive scan of one value per thread across a CTA (warp shuffles + smem).
+//   warp_inclusive_sum  inclusive scan of one value per lane across a warp.
 //   tile_lookback    decoupled look-back over per-tile status words (Merrill & Garland, "Single-pass
 //                    Parallel Prefix Scan with Decoupled Look-back", 2016), replacing the reference's
 //                    three-kernel scan (WVM/src/gpu/queues.cu:69-140): one pass over the data.
@@ -63,26 +63,6 @@ __device__ __forceinline__ uint32_t warp_inclusive_sum(uint32_t v) {
         if (lane >= off) v += o;
     }
     return v;
-}
-
-// Exclusive scan of `v` over the CTA; *total receives the CTA sum. `smem` holds >= 33 words.
-// Every thread of the CTA must call it.
-__device__ __forceinline__ uint32_t block_exclusive_sum(uint32_t v, uint32_t* smem, uint32_t* total) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int nwarps = (blockDim.x + 31) >> 5;
-    const uint32_t inc = warp_inclusive_sum(v);
-    __syncthreads();  // smem may still be read from a previous call
-    if (lane == 31) smem[warp] = inc;
-    __syncthreads();
-    if (warp == 0) {
-        const uint32_t w = lane < nwarps ? smem[lane] : 0u;
-        const uint32_t wi = warp_inclusive_sum(w);
-        if (lane < nwarps) smem[lane] = wi - w;  // exclusive prefix of warp totals
-        if (lane == 31) smem[32] = wi;
-    }
-    __syncthreads();
-    *total = smem[32];
-    return smem[warp] + inc - v;
 }
 
 __device__ __forceinline__ unsigned long long pack_status(unsigned epoch, unsigned flag, uint32_t value) {
