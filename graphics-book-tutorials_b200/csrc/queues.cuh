@@ -33,11 +33,10 @@ __device__ __forceinline__ unsigned long long global_ns() {
     return t;
 }
 
-// Lanes with pred reserve consecutive slots in `items` with ONE atomicAdd per warp; lanes past
-// `capacity` are dropped and counted in *overflow. The whole warp must call it (full mask).
-// Returns the slot, or 0xFFFFFFFF for lanes that did not push or were dropped.
-__device__ __forceinline__ uint32_t queue_push(uint32_t* items, uint32_t* counter, uint32_t capacity,
-                                               uint32_t value, bool pred, uint32_t* overflow) {
+// Lanes with pred reserve consecutive places with ONE atomicAdd per warp; lanes past `capacity` are
+// dropped and counted in *overflow. The whole warp must call it (full mask). Returns the place, or
+// 0xFFFFFFFF for lanes that did not reserve one or were dropped.
+__device__ __forceinline__ uint32_t queue_reserve(uint32_t* counter, uint32_t capacity, bool pred, uint32_t* overflow) {
     const unsigned want = __ballot_sync(kFullMask, pred);
     if (want == 0) return 0xFFFFFFFFu;
     const int lane = threadIdx.x & 31;
@@ -51,7 +50,14 @@ __device__ __forceinline__ uint32_t queue_push(uint32_t* items, uint32_t* counte
         atomicAdd(overflow, 1u);
         return 0xFFFFFFFFu;
     }
-    items[slot] = value;
+    return slot;
+}
+
+// queue_reserve, with `value` written to the place in `items`.
+__device__ __forceinline__ uint32_t queue_push(uint32_t* items, uint32_t* counter, uint32_t capacity,
+                                               uint32_t value, bool pred, uint32_t* overflow) {
+    const uint32_t slot = queue_reserve(counter, capacity, pred, overflow);
+    if (slot != 0xFFFFFFFFu) items[slot] = value;
     return slot;
 }
 
