@@ -22,10 +22,8 @@
 //      state more (icospheres 1280x720x16: 4.2 -> 2.7 ms); the queues remain, as phases C and S, for stage timing
 //      and for the queue-capacity test hook (warp-aggregated pushes, drop-and-count past the capacity).
 //   H  shadow: any-hit traversal of the shadow queue with dynamic fetch; unoccluded contributions
-//      are added to the path radiance (a slot has at most one shadow record per bounce). A single render whose samples have
-//      places of their own in the buffer (LATE) traces them beside the next bounce's extension rays instead, with no
-//      barrier in between: a tail and a barrier less per bounce. 14.6 / 10.3 / 1.18 -> 14.0 / 9.8 / 1.03 ms (icospheres and heightfield
-//      1280x720x16, cornell36 320x180x16).
+//      are added to the path radiance (a slot has at most one shadow record per bounce).
+// Single renders whose samples have places of their own in the buffer run these in two phases instead (wavefront_late).
 // Stage times come from %globaltimer at the barriers (no host synchronisation).
 #include <algorithm>
 #include <cstring>
@@ -53,7 +51,8 @@ struct Control {
     unsigned n_active;
     unsigned n_next;
     unsigned qcount[4];  // lambert, metal, dielectric, shadow
-    unsigned late[2];    // LATE: shadow records of even and odd iterations
+    unsigned late[2];    // wavefront_late: shadow records of even and odd iterations
+    unsigned late_list[2];  // and the slots of the list they leave
     unsigned fetch[2];   // extend, shadow dynamic-fetch cursors
     unsigned unit_next;
     unsigned retired;    // extension rays finished in the current E phase
@@ -388,13 +387,14 @@ constexpr unsigned kRegenTile = kRegenSlots * kWfBlock;
 // Places for the tile's elements with `on` set: *counter grows by their number, and element (k, thread) gets the old value
 // plus the number of elements before it (k first, then thread). Every thread of the CTA calls it; `count` holds a
 // word per k and warp.
-__device__ __forceinline__ void tile_places(const bool (&on)[kRegenSlots], unsigned* counter, unsigned* count,
-                                            unsigned* base, unsigned (&at)[kRegenSlots]) {
+template <int N>
+__device__ __forceinline__ void tile_places(const bool (&on)[N], unsigned* counter, unsigned* count, unsigned* base,
+                                            unsigned (&at)[N]) {
     constexpr int kWarps = kWfBlock / 32;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     __syncthreads();  // count and base may still be read from a previous call
 #pragma unroll
-    for (int k = 0; k < kRegenSlots; ++k) {
+    for (int k = 0; k < N; ++k) {
         const unsigned m = __ballot_sync(kFull, on[k]);
         at[k] = __popc(m & ((1u << lane) - 1u));
         if (lane == 0) count[k * kWarps + warp] = __popc(m);
@@ -402,25 +402,36 @@ __device__ __forceinline__ void tile_places(const bool (&on)[kRegenSlots], unsig
     __syncthreads();
     unsigned total = 0;
 #pragma unroll
-    for (int j = 0; j < kRegenSlots * kWarps; ++j) {
+    for (int j = 0; j < N * kWarps; ++j) {
 #pragma unroll
-        for (int k = 0; k < kRegenSlots; ++k)
+        for (int k = 0; k < N; ++k)
             if (j == k * kWarps + warp) at[k] += total;
         total += count[j];
     }
     if (threadIdx.x == 0) *base = total ? atomicAdd(counter, total) : 0u;
     __syncthreads();
 #pragma unroll
-    for (int k = 0; k < kRegenSlots; ++k) at[k] += *base;
+    for (int k = 0; k < N; ++k) at[k] += *base;
+}
+
+// Adds the threads' counts to the launch's.
+__device__ __forceinline__ void fold_counters(Control* c, unsigned long long n_ext, unsigned long long n_sh, unsigned n_invalid) {
+    for (int off = 16; off > 0; off >>= 1) {
+        n_ext += __shfl_down_sync(kFull, n_ext, off);
+        n_sh += __shfl_down_sync(kFull, n_sh, off);
+        n_invalid += __shfl_down_sync(kFull, n_invalid, off);
+    }
+    if ((threadIdx.x & 31) == 0) {
+        if (n_ext) atomicAdd(&c->ext_rays, n_ext);
+        if (n_sh) atomicAdd(&c->shadow_rays, n_sh);
+        if (n_invalid) atomicAdd(&c->invalid, n_invalid);
+    }
 }
 
 // MINB > 1 caps registers so that MINB CTAs fit an SM (the whole bounce loop is one kernel, so its
 // register count is the largest of any phase's; the traversal phases want the warps more than the
 // shading phases want the registers).
-//
-// LATE (single renders with one place per sample in the buffer, ordered traversal): the shadow rays of an iteration are traced
-// along with the next one's extension rays, without a barrier between the two phases. Direct mode cannot: it folds a finished sample into sums.
-template <bool MULTI, int MINB, bool WIDE, bool LATE>
+template <bool MULTI, int MINB, bool WIDE>
 __global__ void __launch_bounds__(kWfBlock, MINB) wavefront_persistent(const WfArgs a) {
     const Pool& P = a.pool;
     Control* c = P.ctl;
@@ -448,7 +459,6 @@ __global__ void __launch_bounds__(kWfBlock, MINB) wavefront_persistent(const WfA
         if (gtid == 0) {
             c->qcount[0] = c->qcount[1] = c->qcount[2] = c->qcount[3] = 0;
             c->fetch[0] = c->fetch[1] = 0;
-            if (LATE) c->late[iter & 1] = 0;
             c->retired = 0;
         }
         // A CTA takes tiles of kRegenSlots slots per thread: one atomic per tile for the new units and one for the place of
@@ -547,27 +557,22 @@ __global__ void __launch_bounds__(kWfBlock, MINB) wavefront_persistent(const WfA
             c->n_active = n;
             if (n > c->high_water[4]) c->high_water[4] = n;
         }
-        const unsigned n_late = LATE ? *(volatile unsigned*)&c->late[(iter ^ 1) & 1] : 0u;
-        if (n == 0 && n_late == 0) break;
+        if (n == 0) break;
 
         // ---------------- E: extension rays ----------------
         // stragglers may be suspended once 95% of a large phase's rays have finished
-        traverse_phase<false, MULTI, WIDE, LATE>(a, next, n, &c->fetch[0], &n_ext, s_stack, &c->retired,
+        traverse_phase<false, MULTI, WIDE, false>(a, next, n, &c->fetch[0], &n_ext, s_stack, &c->retired,
                                      a.suspend && n >= 4096 ? n - n / 20 : 0xffffffffu);
-        if (LATE) {
-            if (gtid == 0) c->high_water[3] = max(c->high_water[3], n_late);
-            traverse_phase<true, MULTI, WIDE, LATE>(a, nullptr, n_late, &c->fetch[1], &n_sh, s_stack);
-        }
         if (!grid_sync(c, nblocks, 0, &t_last, a.wait_ns)) break;
         if (gtid == 0) c->n_next = 0;  // every CTA has read it; the next regeneration counts from 0
 
-        if (LATE || a.fused) {
+        if (a.fused) {
             // ---------------- C + S in one: classify and shade each path where it is ----------------
             unsigned count[3] = {0, 0, 0};  // per warp, as its material queues would have had them
             for (unsigned base = (unsigned)blockIdx.x * kWfBlock; base < n; base += (unsigned)gthreads) {
                 const unsigned i = base + threadIdx.x;
                 const int slot = i < n ? (int)next[i] : 0;
-                int mat = -1, has = 0, owner = slot;
+                int mat = -1, has = 0;
                 wf::Ray sh;
                 wf::Vec3 contrib{0.f, 0.f, 0.f};
                 if (i < n && P.alive[slot] != 2u) {  // a suspended ray has no hit yet
@@ -593,19 +598,14 @@ __global__ void __launch_bounds__(kWfBlock, MINB) wavefront_persistent(const WfA
                         const bool alive = wf::shade(J.s, ps, f, m, mat, &sh, &contrib, &has);
                         store_path(P, slot, ps);
                         P.alive[slot] = alive ? 1u : 0u;
-                        if (LATE && !alive && has) {
-                            const int4 u = P.unit[slot];
-                            owner = ~((u.y - a.job0.first_sample) * a.job0.film.pixels + u.x);
-                        }
                     }
                 }
 #pragma unroll
                 for (int q = 0; q < 3; ++q) count[q] += __popc(__ballot_sync(kFull, mat == q));
-                const uint32_t at = queue_reserve(LATE ? &c->late[iter & 1] : &c->qcount[3], a.qcap, has != 0, &c->overflow);
+                const uint32_t at = queue_reserve(&c->qcount[3], a.qcap, has != 0, &c->overflow);
                 if (has && at != 0xFFFFFFFFu) {
                     P.sh_dir[at] = make_float4(sh.d.x, sh.d.y, sh.d.z, sh.tmax);
-                    P.sh_c[at] = make_float4(contrib.x, contrib.y, contrib.z, __int_as_float(owner));
-                    if (LATE) P.sh_o[at] = make_float4(sh.o.x, sh.o.y, sh.o.z, 0.f);
+                    P.sh_c[at] = make_float4(contrib.x, contrib.y, contrib.z, __int_as_float(slot));
                 }
             }
             if (lane == 0)
@@ -701,38 +701,159 @@ __global__ void __launch_bounds__(kWfBlock, MINB) wavefront_persistent(const WfA
         if (!a.split_shading && !grid_sync(c, nblocks, 2, &t_last, a.wait_ns)) break;
         }
 
-        if (!LATE) {
-            // ---------------- H: shadow rays ----------------
-            const unsigned nsh = min(*(volatile unsigned*)&c->qcount[3], a.qcap);
-            if (gtid == 0 && nsh > c->high_water[3]) c->high_water[3] = nsh;
-            traverse_phase<true, MULTI, WIDE, LATE>(a, nullptr, nsh, &c->fetch[1], &n_sh, s_stack);
-            if (!grid_sync(c, nblocks, 5, &t_last, a.wait_ns)) break;
-        }
+        // ---------------- H: shadow rays ----------------
+        const unsigned nsh = min(*(volatile unsigned*)&c->qcount[3], a.qcap);
+        if (gtid == 0 && nsh > c->high_water[3]) c->high_water[3] = nsh;
+        traverse_phase<true, MULTI, WIDE, false>(a, nullptr, nsh, &c->fetch[1], &n_sh, s_stack);
+        if (!grid_sync(c, nblocks, 5, &t_last, a.wait_ns)) break;
     }
 
-    // ---- fold counters ----
-    for (int off = 16; off > 0; off >>= 1) {
-        n_ext += __shfl_down_sync(kFull, n_ext, off);
-        n_sh += __shfl_down_sync(kFull, n_sh, off);
-        n_invalid += __shfl_down_sync(kFull, n_invalid, off);
+    fold_counters(c, n_ext, n_sh, n_invalid);
+}
+
+// The form for single renders whose samples have places of their own in the buffer (split mode), with the ordered traversal: two
+// phases per bounce.
+//   E+H   extension rays of this bounce and shadow rays of the last one, with no barrier in between.
+//   C+S+R classify and shade each path; one that ends commits its sample, takes the slot's next one, or another unit, at once (as a
+//         phase of its own that took a barrier and another pass over the list and the radiance). The next list is written tile by tile.
+// A path's radiance is committed before its last shadow ray is traced: that ray's contribution, the last addition to the
+// sample, is made in the buffer. (Direct mode cannot: it folds a finished sample into sums.)
+// Bound by issue at 0.6 of the slots and the waits for path state. Kernel ms, icospheres / heightfield 1280x720x16, cornell36
+// 320x180x16: four phases 14.6 / 10.3 / 1.18; shadow rays beside extension rays 14.0 / 9.8 / 1.01; regeneration in the shading
+// phase 13.4 / 9.4 / 0.89 (with live paths stored after the unit was fetched, so that they spill, 14.0 / 9.9 / 0.90).
+template <int MINB>
+__global__ void __launch_bounds__(kWfBlock, MINB) wavefront_late(const WfArgs a) {
+    const Pool& P = a.pool;
+    const JobDesc& J = a.job0;
+    Control* c = P.ctl;
+    const int lane = threadIdx.x & 31;
+    const unsigned nblocks = gridDim.x + a.bar_extra;  // arrivals that complete a barrier
+    const int gtid = blockIdx.x * blockDim.x + threadIdx.x;
+    const unsigned gthreads = gridDim.x * blockDim.x;
+    __shared__ unsigned s_count[kWfBlock / 32];
+    __shared__ unsigned s_base;
+    __shared__ int s_stack[kStackShared * kWfBlock];
+    unsigned long long t_last = 0;
+    if (blockIdx.x == 0 && threadIdx.x == 0) t_last = global_ns();
+    unsigned long long n_ext = 0, n_sh = 0;
+    unsigned n_invalid = 0;
+    unsigned n = *(volatile unsigned*)&c->n_active, n_late = 0;  // slots in the list, shadow records
+
+    for (unsigned iter = 0;; ++iter) {
+        const int par = iter & 1;
+        const uint32_t* list = P.list[par];
+        uint32_t* next = P.list[par ^ 1];
+        if (iter > 0) {
+            if (gtid == 0) {  // the counters that every CTA read two iterations ago
+                c->late[par] = c->late_list[par] = 0;
+                for (int q = 0; q < 3; ++q) {
+                    c->high_water[q] = max(c->high_water[q], c->qcount[q]);
+                    c->qcount[q] = 0;
+                }
+                c->high_water[3] = max(c->high_water[3], n_late);
+                c->high_water[4] = max(c->high_water[4], n);
+            }
+            traverse_phase<false, false, true, true>(a, list, n, &c->fetch[0], &n_ext, s_stack);
+            traverse_phase<true, false, true, true>(a, nullptr, n_late, &c->fetch[1], &n_sh, s_stack);
+            if (!grid_sync(c, nblocks, 0, &t_last, a.wait_ns)) break;
+            if (gtid == 0) c->fetch[0] = c->fetch[1] = 0;
+        }
+
+        unsigned count[3] = {0, 0, 0};  // per warp, as its material queues would have had them
+        for (unsigned base = (unsigned)blockIdx.x * kWfBlock; base < n; base += gthreads) {
+            const unsigned i = base + threadIdx.x;
+            const int slot = i < n ? (int)list[i] : 0;
+            bool has_path[1] = {false}, need[1] = {i < n && iter == 0}, fresh = false;
+            int mat = -1, has = 0, owner = slot;
+            int4 u = make_int4(0, 0, 0, 0);
+            wf::Ray sh;
+            wf::Vec3 contrib{0.f, 0.f, 0.f};
+            if (i < n && iter > 0) {
+                const float4 hv = P.hit[slot];
+                wf::HitRecord h;
+                h.t = hv.x;
+                h.prim = __float_as_int(hv.y);
+                h.u = hv.z;
+                h.v = hv.w;
+                if (!hit_is_valid(J.s, h)) {
+                    ++n_invalid;
+                    h.prim = -1;  // treated as a miss
+                }
+                wf::PathState ps = load_path(P, slot);
+                wf::Surface f;
+                wf::Material m;
+                mat = wf::classify(J.s, ps, h, J.max_depth, &f, &m);
+                if (mat >= 0) has_path[0] = wf::shade(J.s, ps, f, m, mat, &sh, &contrib, &has);
+                if (has_path[0]) {
+                    store_path(P, slot, ps);
+                } else {
+                    u = P.unit[slot];
+                    const size_t at = sample_slot(u.x, u.y - J.first_sample, J.film.pixels);
+                    J.lbuf[at] = ps.L.x;
+                    J.lbuf[at + 1] = ps.L.y;
+                    J.lbuf[at + 2] = ps.L.z;
+                    owner = ~((u.y - J.first_sample) * J.film.pixels + u.x);
+                    u.y += 1;
+                    fresh = u.y < u.z;
+                    need[0] = !fresh;
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < 3; ++q) count[q] += __popc(__ballot_sync(kFull, mat == q));
+            const uint32_t rec = queue_reserve(&c->late[par], a.qcap, has != 0, &c->overflow);
+            if (has && rec != 0xFFFFFFFFu) {
+                P.sh_dir[rec] = make_float4(sh.d.x, sh.d.y, sh.d.z, sh.tmax);
+                P.sh_c[rec] = make_float4(contrib.x, contrib.y, contrib.z, __int_as_float(owner));
+                P.sh_o[rec] = make_float4(sh.o.x, sh.o.y, sh.o.z, 0.f);
+            }
+            unsigned at[1];
+            tile_places(need, &c->unit_next, s_count, &s_base, at);
+            if (need[0] && at[0] < J.units) {
+                const unsigned pixels = (unsigned)J.film.pixels, k = at[0] / pixels;
+                u.x = (int)(at[0] - k * pixels);
+                u.y = J.first_sample + (int)k * J.chunk;
+                u.z = min(u.y + J.chunk, J.first_sample + J.sample_count);
+                fresh = true;
+            }
+            if (fresh) {
+                P.unit[slot] = u;
+                store_path(P, slot, wf::init_path(J.s, u.x % J.s.width, u.x / J.s.width, (uint32_t)u.y, J.seed));
+                has_path[0] = true;
+            }
+            tile_places(has_path, &c->late_list[par], s_count, &s_base, at);
+            if (has_path[0]) next[at[0]] = (uint32_t)slot;
+        }
+        if (lane == 0)
+            for (int q = 0; q < 3; ++q)
+                if (count[q]) atomicAdd(&c->qcount[q], count[q]);
+        if (!grid_sync(c, nblocks, 1, &t_last, a.wait_ns)) break;
+        n = *(volatile unsigned*)&c->late_list[par];
+        n_late = *(volatile unsigned*)&c->late[par];
+        if (n == 0 && n_late == 0) break;
     }
-    if (lane == 0) {
-        if (n_ext) atomicAdd(&c->ext_rays, n_ext);
-        if (n_sh) atomicAdd(&c->shadow_rays, n_sh);
-        if (n_invalid) atomicAdd(&c->invalid, n_invalid);
-    }
+
+    fold_counters(c, n_ext, n_sh, n_invalid);
 }
 
 using WfKernel = void (*)(const WfArgs);
 
 // The compiled register-cap variants: 0 (none), 6, 8 or 10 CTAs of kWfBlock threads per SM.
-template <bool MULTI, bool WIDE, bool LATE>
+template <bool MULTI, bool WIDE>
 WfKernel wavefront_kernel(int occupancy) {
     switch (occupancy) {
-        case 6: return wavefront_persistent<MULTI, 6, WIDE, LATE>;
-        case 8: return wavefront_persistent<MULTI, 8, WIDE, LATE>;
-        case 10: return wavefront_persistent<MULTI, 10, WIDE, LATE>;
-        default: return wavefront_persistent<MULTI, 1, WIDE, LATE>;
+        case 6: return wavefront_persistent<MULTI, 6, WIDE>;
+        case 8: return wavefront_persistent<MULTI, 8, WIDE>;
+        case 10: return wavefront_persistent<MULTI, 10, WIDE>;
+        default: return wavefront_persistent<MULTI, 1, WIDE>;
+    }
+}
+
+WfKernel wavefront_late_kernel(int occupancy) {
+    switch (occupancy) {
+        case 6: return wavefront_late<6>;
+        case 8: return wavefront_late<8>;
+        case 10: return wavefront_late<10>;
+        default: return wavefront_late<1>;
     }
 }
 
@@ -884,9 +1005,9 @@ WavefrontEngine::WavefrontEngine(int pixels, const WavefrontConfig& cfg) : pixel
         throw Error(WFB_ERR_INVALID_ARGUMENT, "wavefront occupancy target must be 0, 6, 8 or 10");
     for (int w = 0; w < 3; ++w) {
         const int cap_ctas = cfg.occupancy >= 0 ? cfg.occupancy : kWfOccupancy[w];
-        state_->kernel[w] = w ? wavefront_kernel<false, true, false>(cap_ctas) : wavefront_kernel<false, false, false>(cap_ctas);
-        state_->kernel_multi[w] = w ? wavefront_kernel<true, true, false>(cap_ctas) : wavefront_kernel<true, false, false>(cap_ctas);
-        state_->kernel_late[w] = w ? wavefront_kernel<false, true, true>(cap_ctas) : nullptr;
+        state_->kernel[w] = w ? wavefront_kernel<false, true>(cap_ctas) : wavefront_kernel<false, false>(cap_ctas);
+        state_->kernel_multi[w] = w ? wavefront_kernel<true, true>(cap_ctas) : wavefront_kernel<true, false>(cap_ctas);
+        state_->kernel_late[w] = w ? wavefront_late_kernel(cap_ctas) : nullptr;
     }
     // L2 residency: the pool (every field a bounce reads or writes) under a persisting window when
     // it fits the device's persisting set-aside (auto), or whenever asked (a partial window). Last in
