@@ -244,10 +244,11 @@ struct WavefrontConfig {
     bool speculate = true;    // as in MegakernelConfig
 };
 // The defaults for the preorder steps, the ordered traversal, and the ordered traversal over a small tree (kSmallTree). Ordered
-// rays are fetched again sooner than they would trace on with few lanes, and its 64-register form is the faster one
-// (icospheres 1280x720x16 at 10 / 8 / 6 CTAs: 15.9 / 14.6 / 14.9 ms, heightfield 10.9 / 10.3 / 11.0); over a small tree
-// the barriers count more than the latency of the nodes (cornell36 320x180x16: 1.60 / 1.36 / 1.18 ms).
-constexpr int kWfOccupancy[3] = {10, 8, 6}, kWfMinActive[3] = {24, 8, 8}, kWfLeafBatch[3] = {8, 16, 16};
+// rays are fetched again sooner than they would trace on with few lanes (icospheres 1280x720x16 at 4 / 8 / 12 / 16 lanes: 13.68 /
+// 13.28 / 13.32 / 13.59 ms), and the 64-register form is the faster one (8 / 6 CTAs: 13.3 / 13.5 ms, heightfield 9.2 / 9.8; 10 CTAs
+// lost 9% and 6% when the phases were four). Over a small tree the barriers count more than the latency of the nodes
+// (cornell36 320x180x16: 8 / 6 CTAs 1.01 / 0.87 ms) and the end of a phase more than its lanes (8 / 4 lanes: 0.87 / 0.85 ms).
+constexpr int kWfOccupancy[3] = {10, 8, 6}, kWfMinActive[3] = {24, 8, 4}, kWfLeafBatch[3] = {8, 16, 16};
 
 // Launch configuration of a batch or a server: the arm and its knobs.
 struct LaunchConfig {
