@@ -508,7 +508,7 @@ def main():
             "peak_source": peak_kind,
             "bytes_model": "224*ext + 96*shadow + 40 B per sample (path-state bytes a wavefront moves)",
             "ext_rays_per_sample": round(ext_ps, 4), "shadow_rays_per_sample": round(sh_ps, 4),
-            "kernel": "megakernel_wide" if arm == "megakernel" else "wavefront_persistent",
+            "kernel": "megakernel_wide" if arm == "megakernel" else "wavefront_late",
             "kernel_ms": round(kernel_ms, 3),
             "issue_active_frac": prof.get("issue_active_frac"),
             "lanes_per_instr": prof.get("lanes_per_instr"),
