@@ -722,7 +722,7 @@ __global__ void __launch_bounds__(kWfBlock, MINB) wavefront_persistent(const WfA
 //         phase of its own that took a barrier and another pass over the list and the radiance). The next list is written tile by tile.
 // A path's radiance is committed before its last shadow ray is traced: that ray's contribution, the last addition to the
 // sample, is made in the buffer. (Direct mode cannot: it folds a finished sample into sums.)
-// Bound by issue (0.63 of the slots, 18.9 lanes) and the waits for path state (3.4 of 9 stall cycles per issue). Kernel ms, icospheres / heightfield 1280x720x16, cornell36
+// Bound by issue (0.63 of the slots, 18.9 lanes) and the waits for path state (3.4 of 10 stall cycles per issue). Kernel ms, icospheres / heightfield 1280x720x16, cornell36
 // 320x180x16: four phases 14.6 / 10.3 / 1.18; shadow rays beside extension rays 14.0 / 9.8 / 1.01; regeneration in the shading
 // phase 13.4 / 9.4 / 0.89, two node steps per vote 13.3 / 9.2 / 0.85 (with live paths stored after the unit was fetched, so that they spill, 14.0 / 9.9 / 0.90).
 template <int MINB>
