@@ -314,7 +314,7 @@ std::shared_ptr<ResidentScene> upload_scene(const wf::Scene& host) {
 
     // One arena of 256-byte aligned parts, packed in pinned staging and copied once.
     enum { kNodes, kPrims, kSpheres, kTriShade, kTriArea, kMaterials, kLights, kParts };
-    const size_t bytes[kParts] = {(size_t)2 * nn * 16,          (size_t)3 * (np > 0 ? np : 1) * 16,
+    const size_t bytes[kParts] = {(size_t)2 * nn * 16,          (size_t)3 * ((size_t)np + 1) * 16,
                                   (size_t)2 * (ns > 0 ? ns : 1) * 16, (size_t)(nt > 0 ? nt : 1) * 16,
                                   (size_t)(nt > 0 ? nt : 1) * 4,  (size_t)nm * sizeof(wf::Material),
                                   (size_t)4 * (nl > 0 ? nl : 1) * 16};
@@ -337,7 +337,9 @@ std::shared_ptr<ResidentScene> upload_scene(const wf::Scene& host) {
     // Padding, placeholder records of empty parts and unused words are zero, so the arena (and its
     // hash) depends on the scene only.
     for (int k = 0; k < kParts; ++k) std::memset(stage + off[k] + bytes[k], 0, align256(bytes[k]) - bytes[k]);
-    if (np == 0) std::memset(stage + off[kPrims], 0, bytes[kPrims]);
+    // behind the primitives, the empty leaf's record (wide_bvh.cuh)
+    std::memset(stage + off[kPrims] + (size_t)3 * np * 16, 0, 3 * 16);
+    std::memcpy(stage + off[kPrims] + (size_t)3 * np * 16 + 12, &ns, 4);
     if (ns == 0) std::memset(stage + off[kSpheres], 0, bytes[kSpheres]);
     if (nt == 0) {
         std::memset(stage + off[kTriShade], 0, bytes[kTriShade]);
@@ -423,7 +425,7 @@ std::shared_ptr<ResidentScene> upload_scene(const wf::Scene& host) {
     // Behind the packed parts: the chunk hashes and the wide build's control block (read back together), then
     // the wide nodes, at most one per internal node.
     const size_t hash_bytes = align256(n_chunks * 8), ctl_bytes = wide_ctl_bytes();
-    const int wide_capacity = nested ? std::max(1, inner_nodes.load()) : 0;
+    const int wide_capacity = nested && np <= kMaxWidePrims ? std::max(1, inner_nodes.load()) : 0;
     const size_t wide_bytes = (size_t)wide_capacity * kWideFloat4 * sizeof(float4);
     cuda_check(cudaMallocAsync(&rs->arena, total + hash_bytes + ctl_bytes + wide_bytes, 0), "allocate scene");
     rs->bytes = total + wide_bytes;
@@ -443,7 +445,7 @@ std::shared_ptr<ResidentScene> upload_scene(const wf::Scene& host) {
     float4* wide = reinterpret_cast<float4*>(base + total + hash_bytes + ctl_bytes);
     int levels = 0;
     if (wide_capacity)
-        levels = launch_wide_build(d, reinterpret_cast<float4*>(base + off[kPrims]), wide, wide_capacity,
+        levels = launch_wide_build(d, reinterpret_cast<float4*>(base + off[kPrims]), np, wide, wide_capacity,
                                    base + total + hash_bytes, 0, 0, 0);
     std::vector<unsigned long long> hashes((hash_bytes + ctl_bytes) / 8);
     cuda_check(cudaMemcpy(hashes.data(), chunk_hash, hash_bytes + ctl_bytes, cudaMemcpyDeviceToHost), "cudaMemcpy hashes");
@@ -452,7 +454,7 @@ std::shared_ptr<ResidentScene> upload_scene(const wf::Scene& host) {
         unsigned long long* ctl = hashes.data() + hash_bytes / 8;
         bool finished = false;
         while (n_wide = wide_build_result(ctl, levels, &finished), !finished) {
-            levels = launch_wide_build(d, nullptr, wide, wide_capacity, base + total + hash_bytes, levels, 0, 0);
+            levels = launch_wide_build(d, nullptr, np, wide, wide_capacity, base + total + hash_bytes, levels, 0, 0);
             cuda_check(cudaMemcpy(ctl, base + total + hash_bytes, ctl_bytes, cudaMemcpyDeviceToHost), "cudaMemcpy wide build");
         }
     }

@@ -58,8 +58,8 @@ int check_boxes_nested(const std::vector<wf::BvhNode>& nodes);
 // of device memory, whose host copy wide_build_result reads: the number of wide nodes, 0 when the tree keeps the preorder
 // traversal; `finished` false when levels are left.
 size_t wide_ctl_bytes();
-int launch_wide_build(const DevScene& s, float4* prims, float4* wide, int capacity, void* ctl, int first_level,
-                      int levels, cudaStream_t stream);
+int launch_wide_build(const DevScene& s, float4* prims, int n_prims, float4* wide, int capacity, void* ctl,
+                      int first_level, int levels, cudaStream_t stream);
 int wide_build_result(const void* ctl_host, int levels_done, bool* finished);
 // Whether renders of this scene view take the ordered traversal (its tree has wide nodes, and the camera,
 // where rays start, is within the range they cover).

@@ -189,6 +189,7 @@ namespace {
 
 // Host build of the wide tree, as wide_build.cu does it; empty when the tree does not qualify.
 std::vector<float4> host_wide(const std::vector<float4>& nodes, int nn, std::vector<float4>& prims, int ns) {
+    const int empty = empty_leaf((int)(prims.size() / 3) - 1);
     for (int i = 0; i < nn; ++i) {
         const float4 lo = nodes[2 * (size_t)i], hi = nodes[2 * (size_t)i + 1];
         if (!box_in_range(lo, hi)) return {};
@@ -207,7 +208,7 @@ std::vector<float4> host_wide(const std::vector<float4>& nodes, int nn, std::vec
         if (!wide_children(nodes.data(), nn, roots[w], &kids)) return {};
         int codes[kWideArity];
         for (int j = 0; j < kWideArity; ++j) {
-            codes[j] = j < kids.n ? f2i(nodes[2 * (size_t)kids.id[j] + 1].w) : 0;
+            codes[j] = j < kids.n ? f2i(nodes[2 * (size_t)kids.id[j] + 1].w) : empty;
             if (codes[j] < 0) {
                 codes[j] = ~(int)roots.size();
                 roots.push_back(kids.id[j]);
@@ -243,10 +244,11 @@ void traverse_ordered_check(const wf::Scene& host, const float* rays, int n, boo
     if (host.nodes.empty()) throw Error(WFB_ERR_NOT_FINALIZED, "Scene not finalized (no BVH nodes)");
     const int nn = (int)host.nodes.size(), np = (int)host.prim_order.size();
     if (nn >= kNodeHeld) throw Error(WFB_ERR_UNSUPPORTED, "BVH has 2^30 nodes or more");
-    std::vector<float4> nodes(2 * (size_t)nn), prims(3 * (size_t)(np > 0 ? np : 1));
+    std::vector<float4> nodes(2 * (size_t)nn), prims(3 * ((size_t)np + 1), make_float4(0, 0, 0, 0));
     for (int i = 0; i < nn; ++i) pack_node(host, i, &nodes[2 * (size_t)i]);
     for (int j = 0; j < np; ++j) pack_prim(host, j, &prims[3 * (size_t)j]);
     const int ns = (int)host.spheres.size();
+    prims[3 * (size_t)np].w = i2f_bits(ns);  // the empty leaf's record
     std::vector<float4> wide;
     if (check_boxes_nested(host.nodes)) wide = host_wide(nodes, nn, prims, ns);
     for (int k = 0; k < 4; ++k) counts[k] = 0;

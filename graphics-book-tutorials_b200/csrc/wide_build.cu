@@ -51,8 +51,8 @@ __global__ void wide_check_leaves(const float4* __restrict__ nodes, int nn, floa
 constexpr int kTopNodes = 128;
 
 // Wide node `at` of a level whose children are numbered from `next` on.
-__device__ void build_node(const float4* __restrict__ nodes, int nn, float4* wide, int capacity, int at, int next,
-                           int* next_count, WideCtl* ctl) {
+__device__ void build_node(const float4* __restrict__ nodes, int nn, float4* wide, int capacity, int empty, int at,
+                           int next, int* next_count, WideCtl* ctl) {
     float4* rec = wide + (size_t)kWideFloat4 * at;
     const int root = *reinterpret_cast<volatile int*>(rec);
     WideKids kids;
@@ -63,7 +63,7 @@ __device__ void build_node(const float4* __restrict__ nodes, int nn, float4* wid
     int codes[kWideArity], inner = 0;
 #pragma unroll
     for (int j = 0; j < kWideArity; ++j) {
-        codes[j] = j < kids.n ? f2i(nodes[2 * kids.id[j] + 1].w) : 0;
+        codes[j] = j < kids.n ? f2i(nodes[2 * kids.id[j] + 1].w) : empty;
         inner += codes[j] < 0;
     }
     int id = inner ? next + atomicAdd(next_count, inner) : 0;
@@ -82,14 +82,15 @@ __device__ void build_node(const float4* __restrict__ nodes, int nn, float4* wid
 }
 
 // One block: levels from the first on while they hold at most `most` nodes.
-__device__ void build_levels(const float4* __restrict__ nodes, int nn, float4* wide, int capacity, int most, WideCtl* ctl) {
+__device__ void build_levels(const float4* __restrict__ nodes, int nn, float4* wide, int capacity, int empty, int most,
+                             WideCtl* ctl) {
     volatile int* count = ctl->count;
     int begin = 0, level = 0;
     for (; level < kWideMaxLevels; ++level) {
         const int n = count[level];
         if (n == 0 || n > most) break;
         for (int i = threadIdx.x; i < n && begin + i < capacity; i += blockDim.x)
-            build_node(nodes, nn, wide, capacity, begin + i, begin + n, &ctl->count[level + 1], ctl);
+            build_node(nodes, nn, wide, capacity, empty, begin + i, begin + n, &ctl->count[level + 1], ctl);
         __threadfence();
         __syncthreads();
         begin += n;
@@ -97,14 +98,15 @@ __device__ void build_levels(const float4* __restrict__ nodes, int nn, float4* w
     if (threadIdx.x == 0) ctl->top = level;
 }
 
-__global__ void wide_build_top(const float4* __restrict__ nodes, int nn, float4* wide, int capacity, WideCtl* ctl) {
-    build_levels(nodes, nn, wide, capacity, kTopNodes, ctl);
+__global__ void wide_build_top(const float4* __restrict__ nodes, int nn, float4* wide, int capacity, int empty,
+                               WideCtl* ctl) {
+    build_levels(nodes, nn, wide, capacity, empty, kTopNodes, ctl);
 }
 
 // A whole tree of at most kSmallNodes preorder nodes in one block, its nodes in shared memory: leaf check and levels.
 constexpr int kSmallNodes = 1024;
 __global__ void wide_build_small(const float4* __restrict__ global_nodes, int nn, float4* prims, int n_spheres,
-                                 float4* wide, int capacity, WideCtl* ctl) {
+                                 float4* wide, int capacity, int empty, WideCtl* ctl) {
     extern __shared__ float4 nodes[];
     for (int i = threadIdx.x; i < 2 * nn; i += blockDim.x) nodes[i] = global_nodes[i];
     if (threadIdx.x == 0) {
@@ -115,45 +117,46 @@ __global__ void wide_build_small(const float4* __restrict__ global_nodes, int nn
     __syncthreads();
     for (int i = threadIdx.x; i < nn; i += blockDim.x)
         if (!check_leaf(nodes, i, prims, n_spheres)) ctl->bad = 1;
-    build_levels(nodes, nn, wide, capacity, capacity, ctl);
+    build_levels(nodes, nn, wide, capacity, empty, capacity, ctl);
 }
 
 // Level `after_top` of those that wide_build_top left.
-__global__ void wide_build_level(const float4* __restrict__ nodes, int nn, float4* wide, int capacity, int after_top,
-                                 WideCtl* ctl) {
+__global__ void wide_build_level(const float4* __restrict__ nodes, int nn, float4* wide, int capacity, int empty,
+                                 int after_top, WideCtl* ctl) {
     const int level = ctl->top + after_top;
     if (level >= kWideMaxLevels) return;
     int begin = 0;
     for (int l = 0; l < level; ++l) begin += ctl->count[l];
     const int n = ctl->count[level];
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n && begin + i < capacity; i += gridDim.x * blockDim.x)
-        build_node(nodes, nn, wide, capacity, begin + i, begin + n, &ctl->count[level + 1], ctl);
+        build_node(nodes, nn, wide, capacity, empty, begin + i, begin + n, &ctl->count[level + 1], ctl);
 }
 
 }  // namespace
 
 size_t wide_ctl_bytes() { return (sizeof(WideCtl) + 255) & ~(size_t)255; }
 
-int launch_wide_build(const DevScene& s, float4* prims, float4* wide, int capacity, void* ctl_mem, int first_level,
-                      int levels, cudaStream_t stream) {
+int launch_wide_build(const DevScene& s, float4* prims, int n_prims, float4* wide, int capacity, void* ctl_mem,
+                      int first_level, int levels, cudaStream_t stream) {
     WideCtl* ctl = static_cast<WideCtl*>(ctl_mem);
+    const int empty = empty_leaf(n_prims);
     (void)cudaGetLastError();  // the check below is for these launches only
     if (first_level == 0) {
         cuda_check(cudaMemsetAsync(ctl, 0, sizeof(WideCtl), stream), "memset wide build");
         if (s.n_nodes <= kSmallNodes) {
             wide_build_small<<<1, 256, (size_t)s.n_nodes * 32, stream>>>(s.nodes, s.n_nodes, prims, s.n_spheres, wide,
-                                                                         capacity, ctl);
+                                                                         capacity, empty, ctl);
             cuda_check(cudaGetLastError(), "wide build launch");
             return 0;
         }
         wide_check_leaves<<<(s.n_nodes + 255) / 256, 256, 0, stream>>>(s.nodes, s.n_nodes, prims, s.n_spheres, wide, ctl);
-        wide_build_top<<<1, 512, 0, stream>>>(s.nodes, s.n_nodes, wide, capacity, ctl);
+        wide_build_top<<<1, 512, 0, stream>>>(s.nodes, s.n_nodes, wide, capacity, empty, ctl);
         if (levels <= 0) levels = std::max(1, (int)std::ceil(0.62 * std::log2((double)capacity)) - 2);
     }
     if (first_level > 0 && levels <= 0) levels = 8;
     const int grid = std::min((capacity + 63) / 64, 148 * 16);
     for (int l = first_level; l < first_level + levels; ++l)
-        wide_build_level<<<grid, 64, 0, stream>>>(s.nodes, s.n_nodes, wide, capacity, l, ctl);
+        wide_build_level<<<grid, 64, 0, stream>>>(s.nodes, s.n_nodes, wide, capacity, empty, l, ctl);
     cuda_check(cudaGetLastError(), "wide build launch");
     return first_level + levels;
 }

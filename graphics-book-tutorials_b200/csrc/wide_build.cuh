@@ -94,7 +94,7 @@ WF_HD bool wide_children(const float4* nodes, int nn, int root, WideKids* out) {
 
 // Writes the wide node: the grid covers the children's boxes with a margin at both ends, and each plane is
 // the nearest grid plane outside the box plane by kPlaneMargin steps or more (less the rounding of the position in steps,
-// 255 * 2^-22 of one, which is far below the margin). codes[] as in the node layout, 0 for slots without a child.
+// 255 * 2^-22 of one, which is far below the margin). codes[] as in the node layout.
 WF_HD void wide_write(const float4* nodes, const WideKids& kids, const int (&codes)[kWideArity], float4* out) {
     const int k = kids.n;
     unsigned lo_q[3] = {~0u, ~0u, ~0u}, hi_q[3] = {0u, 0u, 0u};  // unused slots: inside out
