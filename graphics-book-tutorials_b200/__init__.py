@@ -473,7 +473,9 @@ class GpuRenderer:
         return int(load_library().wfb_renderer_l2_window_bytes(self._h))
 
     def set_speculation(self, on: bool) -> None:
-        """Speculative traversal in both arms (on by default); films are the same bits either way."""
+        """Speculative and ordered traversal in both arms (on by default). Off, every ray takes the plain preorder
+        steps; on, films are the same bits but for rays that graze a triangle's plane so closely that its reported
+        hit lies in front of its own leaf's box by more than 1/1024 (csrc/wide_bvh.cuh)."""
         _check(load_library().wfb_renderer_set_speculation(self._h, int(bool(on))))
 
     def apply_tuning(self, tuning: "TuneResult") -> None:

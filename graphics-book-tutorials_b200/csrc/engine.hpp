@@ -297,7 +297,7 @@ public:
     void set_l2_residency(int mode);
     // Bytes of the wavefront pool under the window (0: none, or a megakernel renderer).
     uint64_t l2_window_bytes() const;
-    // Speculative traversal in both arms (box_step): films are the same bits either way.
+    // Speculative and ordered traversal in both arms (box_step, wide_bvh.cuh); off: the plain preorder steps.
     void set_speculation(bool on);
 
 private:

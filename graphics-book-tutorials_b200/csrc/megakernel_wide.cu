@@ -1,7 +1,8 @@
 // Persistent megakernel over the ordered traversal (wide_bvh.cuh): the kernel of every scene whose tree has wide nodes.
 //
 // Work units, jobs, film order, the order of a path's rays and the estimator steps are those of
-// megakernel_persistent (megakernel.cu); the films are the same bits. What differs, and what it is worth (B200,
+// megakernel_persistent (megakernel.cu); the films are the same bits, but for the hits that kCullSlack (wide_bvh.cuh)
+// leaves open. What differs, and what it is worth (B200,
 // icospheres / heightfield 1280x720x16, cornell36 320x180x16; the preorder kernel takes 22.9 / 12.3 / 0.82 ms):
 //
 //  * Instruction issue bounds it (0.70 of the slots, 15.5 lanes per instruction; DRAM idle): a warp executes about 800

@@ -10,7 +10,8 @@
 // the megakernel) and, when its path ends, regenerates the next sample of the same pixel or takes a
 // new unit: paths in flight stay constant until the work runs out. Film sums are kept per slot in
 // sample order (direct mode) or per (pixel, sample) in a buffer committed in order afterwards
-// (split mode), so the film is bit-identical to every arm.
+// (split mode), so the film is bit-identical to every arm's over the same hits (those of the ordered traversal have the one
+// exception of wide_bvh.cuh).
 //
 // One bounce = four phases separated by grid barriers (bounded spins, error flag on timeout):
 //   R  regenerate + compact: ended slots commit their sample and start the next one (or fetch a

@@ -30,7 +30,7 @@ public:
     int capacity() const { return capacity_; }
     // Bytes of the pool under a persisting L2 access-policy window on every launch (0: none).
     size_t l2_window_bytes() const;
-    // Speculative traversal on or off for the following launches (box_step; same films either way).
+    // Speculative and ordered traversal on or off for the following launches (box_step, wide_bvh.cuh).
     void set_speculate(bool on) { cfg_.speculate = on; }
 
 private:

@@ -193,11 +193,15 @@ int wfb_renderer_configure(wfb_renderer_t r, int block, int blocks_per_sm, int m
 int wfb_renderer_set_l2_residency(wfb_renderer_t r, int mode);
 /* Bytes of the wavefront pool under the persisting window (0: none). */
 uint64_t wfb_renderer_l2_window_bytes(wfb_renderer_t r);
-/* Speculative traversal in both arms (no reference counterpart; on by default): a lane whose ray
- * holds a leaf still to test goes on with box tests, and the next leaf it reaches is tested again
- * once the first is done, so leaves are still entered in the reference's order and films are the
- * same bits either way (WVM/include/wf/bvh.hpp:91-116). Closest-hit rays speculate only on a BVH
- * whose boxes nest (wfb_scene_boxes_nested) and whose direction has no zero component. */
+/* Speculative and ordered traversal in both arms (no reference counterpart; on by default).
+ * Trees that qualify (nested boxes, primitives inside their leaf's box, one leaf per primitive entry)
+ * take an ordered traversal: nearest child first, with the hit preorder traversal returns
+ * (WVM/include/wf/bvh.hpp:91-116) except where a primitive reports a t that lies in front of its own
+ * leaf's box by more than 1/1024: a triangle whose plane the ray all but lies in, or a sliver, with
+ * another surface in the gap. On other trees a lane whose ray holds a leaf still to test goes on with
+ * box tests, and the next leaf it reaches is tested again once the first is done, so leaves are entered
+ * in the reference's order; closest-hit rays do so only on a BVH whose boxes nest (wfb_scene_boxes_nested)
+ * and with a direction that has no zero component. Off: the plain preorder steps, without exception. */
 int wfb_renderer_set_speculation(wfb_renderer_t r, int on);
 int wfb_renderer_width(wfb_renderer_t r);
 int wfb_renderer_height(wfb_renderer_t r);
