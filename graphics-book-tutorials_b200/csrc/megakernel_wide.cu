@@ -18,6 +18,7 @@
 //    with the stacks). 7 and 6 CTAs spill less but leave the latency of the node chase open (13.0 / 8.7 at 7).
 //  * A launch with fewer units than lanes spreads over all warps (64x36x1: 0.162 -> 0.088 ms).
 #include <algorithm>
+#include "counts.hpp"
 #include "engine.hpp"
 #include "wide_lane.cuh"
 #include "../../include/wfb200.h"
@@ -74,9 +75,9 @@ __global__ void __launch_bounds__(kBlock, kCtas) megakernel_wide(const WideArgs 
     int kind = kNoPath;
     // A launch with fewer units than lanes spreads them over all warps, the first lanes of each: a warp of few rays ends
     // sooner than one of 32 that diverge.
-    const unsigned warps = gridDim.x * (kBlock / 32), share = (total_units + warps - 1) / warps;
+    const unsigned share = warp_share(total_units, gridDim.x * (kBlock / 32));
     bool out_of_work = (unsigned)lane >= share;
-    const int min_active = min(a.min_active, (int)min((share + 1) / 2, 32u));
+    const int min_active = spread_min_active(a.min_active, share);
     wf::Vec3 o{0.f, 0.f, 0.f};
     TravRay ray;
     ray.d = ray.inv_d = wf::Vec3{0.f, 0.f, 0.f};

@@ -7,6 +7,7 @@
 // it by CTAs that are already running: the look-back always makes progress.
 #include <atomic>
 #include <cstring>
+#include "counts.hpp"
 #include "engine.hpp"
 #include "queues.cuh"
 #include "queues.hpp"
@@ -169,7 +170,7 @@ void launch_scan(const uint32_t* in, const uint32_t* values, uint32_t* out, int 
     const bool aligned = (bits & 15) == 0;
     const bool large = n >= kLargeScan;
     const int tile = large ? kTileElements<kLargeChunks> : kSmallTile;
-    const int tiles = (n + tile - 1) / tile;
+    const int tiles = scan_tile_count(n, tile);
     const auto kernel = large ? scan_tiles<MODE, kLargeChunks> : scan_tiles<MODE, 1>;
     (void)cudaGetLastError();  // the check below is for this launch only
     kernel<<<tiles, kScanBlock, 0, stream>>>(in, values, out, n, total, ws.status, ws.ticket, first, aligned, epoch,
