@@ -759,8 +759,14 @@ __global__ void __launch_bounds__(kWfBlock, MINB) wavefront_late(const WfArgs a)
                 c->high_water[4] = max(c->high_water[4], n);
             }
             traverse_phase<false, false, true, true>(a, list, n, &c->fetch[0], &n_ext, s_stack);
+            // stage times: extension until the first CTA's first warp has no more such rays, shadow rays from there to the barrier
+            if (gtid == 0) {
+                const unsigned long long now = global_ns();
+                c->stage_ns[0] += now - t_last;
+                t_last = now;
+            }
             traverse_phase<true, false, true, true>(a, nullptr, n_late, &c->fetch[1], &n_sh, s_stack);
-            if (!grid_sync(c, nblocks, 0, &t_last, a.wait_ns)) break;
+            if (!grid_sync(c, nblocks, 5, &t_last, a.wait_ns)) break;
             if (gtid == 0) c->fetch[0] = c->fetch[1] = 0;
         }
 

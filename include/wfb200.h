@@ -143,7 +143,11 @@ typedef struct {
     int64_t queue_overflows;
     int64_t invalid_hits;
     uint64_t peak_vram_bytes;
-    double stage_ms[8]; /* extend, classify, lambert, metal, dielectric, shadow, compact, other */
+    /* extend, classify, lambert, metal, dielectric, shadow, compact, other (wavefront). With stage_timing the
+     * stages run apart, material by material; without it, as renders run them: classify then holds the shading
+     * (and the regeneration, compact 0, where samples have places of their own in the sample buffer and the
+     * tree the ordered traversal; extend and shadow, one phase there, are told apart by the first CTA's clock) */
+    double stage_ms[8];
     uint64_t node_visits; /* megakernel, with count_rays: BVH nodes visited (box tests) */
     uint64_t prim_tests;  /* megakernel, with count_rays: primitive intersection tests */
     uint64_t kernel_launches; /* kernels of this library launched by the call */
