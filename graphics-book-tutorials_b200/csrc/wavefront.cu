@@ -842,6 +842,8 @@ __global__ void __launch_bounds__(kWfBlock, MINB) wavefront_late(const WfArgs a)
         n_late = *(volatile unsigned*)&c->late[par];
         if (n == 0 && n_late == 0) break;
     }
+    if (gtid == 0)  // the last iteration's, which no other one folds
+        for (int q = 0; q < 3; ++q) c->high_water[q] = max(c->high_water[q], *(volatile unsigned*)&c->qcount[q]);
 
     fold_counters(c, n_ext, n_sh, n_invalid);
 }

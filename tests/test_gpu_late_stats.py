@@ -2,6 +2,8 @@
 those of the barriered phases, which stage timing runs."""
 import pytest
 
+from test_ordered_traversal import _ball_scene
+
 pytestmark = pytest.mark.gpu
 
 
@@ -13,3 +15,17 @@ def test_stage_times_of_an_ordinary_render(wfb, scene):
     r.render(wfb.RenderParams(spp=8, seed=3, max_depth=8), st)
     assert st.stages["extend"] > 0 and st.stages["shadow"] > 0 and st.stages["classify"] > 0
     assert sum(st.stages.values()) <= st.render_ms
+
+
+def test_queue_high_water_counts_the_last_bounce(wfb):
+    """Two paths at a time through balls of every material: where the last bounce of a film is the only one of its material (the
+    path ends in it), the material's high-water mark still counts it."""
+    _, arrays = _ball_scene(wfb, 300, 3)
+    r = wfb.GpuRenderer(wfb.Scene.from_arrays(dict(arrays, width=1, height=1)), wfb.WAVEFRONT)
+    marks = {False: [], True: []}
+    for seed in range(1, 301):
+        for staged in marks:
+            st = wfb.RenderStats()
+            r.render(wfb.RenderParams(spp=2, seed=seed, max_depth=8, stage_timing=staged), st)
+            marks[staged].append(tuple(st.queue_high_water[:3]))
+    assert marks[False] == marks[True]
