@@ -205,6 +205,7 @@ def load_library(path: str = LIB_PATH) -> ctypes.CDLL:
         "wfb_renderer_set_l2_residency": (i32, [vp, i32]),
         "wfb_renderer_set_speculation": (i32, [vp, i32]),
         "wfb_scene_boxes_nested": (i32, [vp, ctypes.POINTER(ctypes.c_int)]),
+        "wfb_scene_wide_nodes": (i32, [vp, ctypes.POINTER(ctypes.c_int)]),
         "wfb_test_traverse": (i32, [vp, vp, i32, i32, i32, i32, i32, vp]),
         "wfb_test_traverse_wide": (i32, [vp, vp, i32, i32, vp, vp]),
         "wfb_test_traverse_ordered": (i32, [vp, vp, i32, i32, vp, vp]),
@@ -334,6 +335,12 @@ class Scene:
         v = ctypes.c_int(0)
         _check(load_library().wfb_scene_boxes_nested(self._h, ctypes.byref(v)))
         return bool(v.value)
+
+    def wide_nodes(self) -> int:
+        """Nodes of the wide tree that the device built (uploads the scene); 0 when renders traverse in preorder."""
+        v = ctypes.c_int(0)
+        _check(load_library().wfb_scene_wide_nodes(self._h, ctypes.byref(v)))
+        return v.value
 
     def info(self) -> SceneInfo:
         inf = SceneInfo()

@@ -305,6 +305,14 @@ int wfb_scene_boxes_nested(wfb_scene_t s, int* nested) {
     });
 }
 
+int wfb_scene_wide_nodes(wfb_scene_t s, int* nodes) {
+    return guarded([&] {
+        need(s && nodes, "null argument");
+        if (s->host.nodes.empty()) throw wfb::Error(WFB_ERR_NOT_FINALIZED, "Scene not finalized (no BVH nodes)");
+        *nodes = s->get_resident()->wide_nodes;
+    });
+}
+
 int wfb_scene_export(wfb_scene_t s, void* spheres, float* vertices, int* triangles, void* materials,
                      void* nodes, int* prim_order, void* lights) {
     return guarded([&] {

@@ -459,6 +459,7 @@ std::shared_ptr<ResidentScene> upload_scene(const wf::Scene& host) {
         }
     }
     d.wide = n_wide > 0 ? wide : nullptr;
+    rs->wide_nodes = n_wide;
     hashes.resize(n_chunks);
     uint64_t key = 0x6A09E667F3BCC909ull ^ total;
     for (unsigned long long h : hashes) key = fold(key, h);

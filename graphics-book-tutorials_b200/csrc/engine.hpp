@@ -36,6 +36,7 @@ struct ResidentScene {
     DevScene dev{};  // device pointers into `arena`; camera/resolution are the host defaults
     void* arena = nullptr;
     uint64_t bytes = 0;
+    int wide_nodes = 0;         // nodes of the wide tree (wide_bvh.cuh); 0: the scene keeps the preorder traversal
     uint64_t content_key = 0;   // hash of the packed arena, environment and default camera
     int device = -1;
     // Recorded after work that reads the arena on a caller's stream and returns without waiting

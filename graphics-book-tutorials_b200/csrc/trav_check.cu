@@ -203,7 +203,12 @@ std::vector<float4> host_wide(const std::vector<float4>& nodes, int nn, std::vec
     }
     std::vector<int> roots{0};
     std::vector<float4> wide;
-    for (size_t w = 0; w < roots.size(); ++w) {
+    size_t level_end = 1;  // nodes are numbered level by level
+    for (size_t w = 0, level = 1; w < roots.size(); ++w) {
+        if (w == level_end) {
+            if (++level > kWideMaxLevels) return {};
+            level_end = roots.size();
+        }
         WideKids kids;
         if (!wide_children(nodes.data(), nn, roots[w], &kids)) return {};
         int codes[kWideArity];

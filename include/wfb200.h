@@ -106,6 +106,9 @@ int wfb_scene_info_get(wfb_scene_t scene, wfb_scene_info* info);
  * box of each node whose subtree -- the nodes before its skip link -- holds it): the condition for
  * exact speculative closest-hit traversal (wfb_renderer_set_speculation). Host only. */
 int wfb_scene_boxes_nested(wfb_scene_t scene, int* nested);
+/* Nodes of the wide tree built on the device at upload (uploads the scene if it is not resident); 0: the tree
+ * does not qualify and its renders traverse in preorder. */
+int wfb_scene_wide_nodes(wfb_scene_t scene, int* nodes);
 /* Copies the finalized host arrays into caller buffers sized from wfb_scene_info (any pointer
  * may be NULL to skip that array). */
 int wfb_scene_export(wfb_scene_t scene, void* spheres, float* vertices, int* triangles,

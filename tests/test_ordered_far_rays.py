@@ -61,6 +61,7 @@ def test_far_rays_equal_preorder(wfb, orc, half, distance, anyhit):
 @pytest.mark.parametrize("half,distance", FAR)
 def test_films_seen_from_far_away(wfb, half, distance):
     scene, _ = _cluster(wfb, half, distance)
+    assert scene.wide_nodes() > 0
     for mode in (wfb.MEGAKERNEL, wfb.WAVEFRONT):
         films = []
         for on in (True, False):
