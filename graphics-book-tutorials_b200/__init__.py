@@ -104,7 +104,7 @@ STAGE_NAMES = ("extend", "classify", "shade_lambert", "shade_metal", "shade_diel
 class _CTuneResult(ctypes.Structure):
     _fields_ = [("mode", ctypes.c_int), ("block", ctypes.c_int), ("occupancy", ctypes.c_int),
                 ("min_active", ctypes.c_int), ("leaf_batch", ctypes.c_int), ("paths_in_flight", ctypes.c_int),
-                ("wf_min_active", ctypes.c_int),
+                ("wf_min_active", ctypes.c_int), ("keep_defaults", ctypes.c_int),
                 ("msamples_s", ctypes.c_double),
                 ("megakernel_msamples_s", ctypes.c_double), ("wavefront_msamples_s", ctypes.c_double),
                 ("candidates", ctypes.c_int), ("wf_occupancy", ctypes.c_int)]
@@ -517,13 +517,14 @@ class TuneResult:
     candidates: int
     wf_occupancy: int
     _c: _CTuneResult = field(repr=False, default=None)
+    keep_defaults: int = 0  # 1: the megakernel's defaults are applied, not its knobs above; 2: the wavefront's
 
     def as_dict(self) -> dict:
         return {"arm": "megakernel" if self.mode == MEGAKERNEL else "wavefront",
                 "megakernel": {"block": self.block, "occupancy": self.occupancy, "min_active": self.min_active,
-                               "leaf_batch": self.leaf_batch},
+                               "leaf_batch": self.leaf_batch, "defaults_kept": bool(self.keep_defaults & 1)},
                 "wavefront": {"paths_in_flight": self.paths_in_flight, "min_active": self.wf_min_active,
-                              "occupancy": self.wf_occupancy},
+                              "occupancy": self.wf_occupancy, "defaults_kept": bool(self.keep_defaults & 2)},
                 "msamples_s": round(self.msamples_s, 2),
                 "megakernel_msamples_s": round(self.megakernel_msamples_s, 2),
                 "wavefront_msamples_s": round(self.wavefront_msamples_s, 2), "candidates": self.candidates}
@@ -538,7 +539,7 @@ def autotune(scene: Scene, width: int, height: int, probe_spp: int = 2, max_dept
                                        1 if try_wavefront else 0, ctypes.byref(c)))
     return TuneResult(c.mode, c.block, c.occupancy, c.min_active, c.leaf_batch, c.paths_in_flight, c.wf_min_active,
                       c.msamples_s,
-                      c.megakernel_msamples_s, c.wavefront_msamples_s, c.candidates, c.wf_occupancy, c)
+                      c.megakernel_msamples_s, c.wavefront_msamples_s, c.candidates, c.wf_occupancy, c, c.keep_defaults)
 
 
 def compare_results(a: RenderResult, b: RenderResult) -> dict:

@@ -3,20 +3,15 @@
 //
 // Candidates are rendered for `probe_spp` samples at the target resolution, each once to warm up
 // and twice timed with CUDA events (the faster run counts); the fastest configuration wins. Every candidate
-// renders the same film bits (launch knobs never change the arithmetic), so tuning is purely a
+// renders the same film bits (launch knobs never change a lane's arithmetic), so tuning is purely a
 // speed decision. Results are cached per (scene content, camera, width, height, probe_spp,
 // max_depth); the content key is the uploaded arena's hash (upload_scene).
 // The result holds the best knobs of each arm, so a renderer of either arm can apply it.
-//   megakernel: stage 1, (block, occupancy target) in {(128,10), (128,8), (128,6), (128,0), (64,0), (256,0)}
-//               x min_active in {8, 16, 24} at leaf_batch 8; stage 2, the stage-1 winner with
-//               leaf_batch in {4, 12, 16, 32}; stage 3, min_active 4 either side of the winner
-//   wavefront:  stage 1, paths in flight in {the largest pool that fits the persisting L2 set-aside
-//               (its launches carry a persisting access-policy window), 2M, 4M, 8M, 16M} (each capped at 64
-//               per pixel, duplicates probed once) x register cap {10, 8} CTAs per SM; stage 2,
-//               min_active {16, 24}; probed with enough samples that the largest pool turns over about
-//               twice (8 to 64 per pixel). Queue capacity is
-//               not a knob: every queue is sized to the pool, so none can drop a path (the
-//               reference's capacity knob exists to test overflow, WVM/src/gpu/wavefront.cu:279-280).
+// Which configurations are timed: tune_search.hpp. Wavefront probes take paths in flight from {the largest pool that fits the
+// persisting L2 set-aside (its launches carry a persisting access-policy window), 2M, 4M, 8M, 16M} (each capped at 64
+// per pixel, duplicates probed once), with enough samples that the largest pool turns over about twice (8 to 64 per
+// pixel). Queue capacity is not a knob: every queue is sized to the pool, so none can drop a path (the
+// reference's capacity knob exists to test overflow, WVM/src/gpu/wavefront.cu:279-280).
 #include <algorithm>
 #include <cstring>
 #include <map>
@@ -68,46 +63,14 @@ TuneResult autotune(const std::shared_ptr<ResidentScene>& scene, const wf::Camer
     TuneResult best;
     best.mode = WFB_MODE_MEGAKERNEL;
     double mk_ms = 1e300, wf_ms = 1e300;
+    const bool ordered = wide_usable(with_camera(scene->dev, cam, width, height));
     {
         Renderer r(scene, wf::GpuMode::Megakernel);
         r.set_camera(cam, width, height);
-        const int shapes[][2] = {{128, 10}, {128, 8}, {128, 6}, {128, 0}, {64, 0}, {256, 0}};
-        const int actives[] = {8, 16, 24};
-        best.leaf_batch = 8;
-        for (const auto& sh : shapes)
-            for (int ma : actives) {
-                r.configure(sh[0], 0, ma, 0, -1, sh[1], best.leaf_batch);
-                const double ms = measure(r, p);
-                best.candidates++;
-                if (ms < mk_ms) {
-                    mk_ms = ms;
-                    best.block = sh[0];
-                    best.occupancy = sh[1];
-                    best.min_active = ma;
-                }
-            }
-        const int batches[] = {4, 12, 16, 32};
-        for (int lb : batches) {
-            r.configure(best.block, 0, best.min_active, 0, -1, best.occupancy, lb);
-            const double ms = measure(r, p);
-            best.candidates++;
-            if (ms < mk_ms) {
-                mk_ms = ms;
-                best.leaf_batch = lb;
-            }
-        }
-        // stage 3: min_active 4 either side of the winner (the steps of stage 1 are 8 apart)
-        const int ma0 = best.min_active;
-        for (int ma : {ma0 - 4, ma0 + 4}) {
-            if (ma < 1 || ma > 32) continue;
-            r.configure(best.block, 0, ma, 0, -1, best.occupancy, best.leaf_batch);
-            const double ms = measure(r, p);
-            best.candidates++;
-            if (ms < mk_ms) {
-                mk_ms = ms;
-                best.min_active = ma;
-            }
-        }
+        mk_ms = search_megakernel(ordered, [&](const MegakernelKnobs& k) {
+            r.configure(k.block, 0, k.min_active, 0, -1, k.occupancy, k.leaf_batch);
+            return measure(r, p);
+        }, best);
     }
     if (try_wavefront) {
         int dev = 0;
@@ -129,29 +92,10 @@ TuneResult autotune(const std::shared_ptr<ResidentScene>& scene, const wf::Camer
         const double samples_w = (double)width * height * pw.sample_count;
         Renderer r(scene, wf::GpuMode::Wavefront);
         r.set_camera(cam, width, height);
-        // stage 1: pool x register cap at one min_active; stage 2: min_active
-        best.wf_min_active = wide_usable(scene->dev) ? 16 : 24;
-        const int occs[] = {10, 8};
-        for (int pool : pools)
-            for (int occ : occs) {
-                r.configure(-1, -1, best.wf_min_active, -1, pool, occ);
-                const double ms = measure(r, pw) * samples / samples_w;  // per probe_spp samples
-                best.candidates++;
-                if (ms < wf_ms) {
-                    wf_ms = ms;
-                    best.paths_in_flight = pool;
-                    best.wf_occupancy = occ;
-                }
-            }
-        for (int ma : {16, 24}) {
-            r.configure(-1, -1, ma, -1, best.paths_in_flight, best.wf_occupancy);
-            const double ms = measure(r, pw) * samples / samples_w;
-            best.candidates++;
-            if (ms < wf_ms) {
-                wf_ms = ms;
-                best.wf_min_active = ma;
-            }
-        }
+        wf_ms = search_wavefront(ordered, pools, [&](int pool, const WavefrontKnobs& k) {
+            r.configure(-1, -1, k.min_active, -1, pool, k.occupancy);
+            return measure(r, pw) * samples / samples_w;  // per probe_spp samples
+        }, best);
     }
     best.megakernel_msamples_s = samples / mk_ms / 1e3;
     if (try_wavefront) best.wavefront_msamples_s = samples / wf_ms / 1e3;
@@ -163,12 +107,15 @@ TuneResult autotune(const std::shared_ptr<ResidentScene>& scene, const wf::Camer
 }
 
 void apply_tuning(Renderer& r, const TuneResult& t) {
-    if (r.mode() == wf::GpuMode::Megakernel)
+    const int pool = t.paths_in_flight > 0 ? t.paths_in_flight : -1;
+    if (t.keep_defaults & (r.mode() == wf::GpuMode::Megakernel ? kTuneMegakernel : kTuneWavefront)) {
+        r.default_knobs(pool);
+    } else if (r.mode() == wf::GpuMode::Megakernel) {
         r.configure(t.block > 0 ? t.block : -1, -1, t.min_active > 0 ? t.min_active : -1, -1, -1,
                     t.occupancy >= 0 ? t.occupancy : -1, t.leaf_batch > 0 ? t.leaf_batch : -1);
-    else
-        r.configure(-1, -1, t.wf_min_active > 0 ? t.wf_min_active : -1, -1,
-                    t.paths_in_flight > 0 ? t.paths_in_flight : -1, t.wf_occupancy >= 0 ? t.wf_occupancy : -1);
+    } else {
+        r.configure(-1, -1, t.wf_min_active > 0 ? t.wf_min_active : -1, -1, pool, t.wf_occupancy >= 0 ? t.wf_occupancy : -1);
+    }
 }
 
 }  // namespace wfb

@@ -504,6 +504,7 @@ int wfb_autotune(wfb_scene_t scene, int width, int height, int probe_spp, int ma
         out->paths_in_flight = t.paths_in_flight;
         out->wf_min_active = t.wf_min_active;
         out->wf_occupancy = t.wf_occupancy;
+        out->keep_defaults = t.keep_defaults;
         out->msamples_s = t.msamples_s;
         out->megakernel_msamples_s = t.megakernel_msamples_s;
         out->wavefront_msamples_s = t.wavefront_msamples_s;
@@ -523,6 +524,7 @@ int wfb_renderer_apply_tuning(wfb_renderer_t r, const wfb_tune_result* t) {
         tr.paths_in_flight = t->paths_in_flight;
         tr.wf_min_active = t->wf_min_active;
         tr.wf_occupancy = t->wf_occupancy;
+        tr.keep_defaults = t->keep_defaults;
         wfb::apply_tuning(*r->r, tr);
     });
 }

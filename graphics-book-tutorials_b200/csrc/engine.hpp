@@ -294,6 +294,8 @@ public:
     // Values < 0 keep the current setting (block and min_active also keep on 0).
     void configure(int block, int blocks_per_sm, int min_active, int split_chunks, int paths_in_flight,
                    int occupancy, int leaf_batch = -1);
+    // The arm's block, occupancy, min_active and leaf_batch back to their defaults; paths_in_flight < 0 keeps the pool.
+    void default_knobs(int paths_in_flight);
     // Wavefront pool under a persisting L2 window: -1 when it fits the set-aside, 0 never, 1 always.
     void set_l2_residency(int mode);
     // Bytes of the wavefront pool under the window (0: none, or a megakernel renderer).

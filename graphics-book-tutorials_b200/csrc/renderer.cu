@@ -339,6 +339,23 @@ void Renderer::configure(int block, int blocks_per_sm, int min_active, int split
     }
 }
 
+void Renderer::default_knobs(int paths_in_flight) {
+    const MegakernelConfig mk{};
+    mk_cfg_.block = mk.block;
+    mk_cfg_.occupancy = mk.occupancy;
+    mk_cfg_.min_active = mk.min_active;
+    mk_cfg_.leaf_batch = mk.leaf_batch;
+    const WavefrontConfig wf{};
+    wf_cfg_.occupancy = wf.occupancy;
+    wf_cfg_.min_active = wf.min_active;
+    wf_cfg_.leaf_batch = wf.leaf_batch;
+    if (paths_in_flight > 0) wf_cfg_.paths_in_flight = paths_in_flight;
+    if (mode_ != wf::GpuMode::Wavefront) return;
+    cuda_check(cudaStreamSynchronize(stream_), "cudaStreamSynchronize");
+    wf_.reset();
+    wf_ = std::make_unique<Wavefront>(pixels(), wf_cfg_);
+}
+
 void Renderer::set_l2_residency(int mode) {
     wf_cfg_.l2_persist = mode < 0 ? -1 : (mode > 0 ? 1 : 0);
     if (mode_ != wf::GpuMode::Wavefront) return;

@@ -219,11 +219,13 @@ int wfb_renderer_destroy(wfb_renderer_t r);
  * Measures launch configurations of both arms on `scene` (its camera) at width x height for
  * probe_spp samples: the faster arm (mode), the best megakernel block / occupancy target /
  * min_active / leaf_batch and the best wavefront paths in flight / min_active (0 when the
- * wavefront was not tried). Cached per scene content and size. */
+ * wavefront was not tried). An arm whose defaults are as fast as its best knobs has its bit in keep_defaults: applying the
+ * result then sets its knobs (all but paths_in_flight) to their defaults. Cached per scene content and size. */
 typedef struct {
     int mode;
     int block, occupancy, min_active, leaf_batch;
     int paths_in_flight, wf_min_active;
+    int keep_defaults; /* 1: the megakernel's, 2: the wavefront's (in what was padding: set it to 0 in a result of your own) */
     double msamples_s, megakernel_msamples_s, wavefront_msamples_s;
     int candidates;
     int wf_occupancy; /* wavefront register cap: 0, 6, 8 or 10 CTAs of 128 threads per SM */
