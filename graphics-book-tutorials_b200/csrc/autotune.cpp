@@ -96,6 +96,13 @@ TuneResult autotune(const std::shared_ptr<ResidentScene>& scene, const wf::Camer
             r.configure(-1, -1, k.min_active, -1, pool, k.occupancy);
             return measure(r, pw) * samples / samples_w;  // per probe_spp samples
         }, best);
+        // The arms are compared over renders of one length: the megakernel's short probes, which rank its own knobs, end in a
+        // tail that the wavefront's longer ones spread (cornell36 320x180: 1,088 Msamples/s at 8 samples per pixel,
+        // 1,778 at 64; icospheres 1280x720: 1,121 at 8, 1,166 at 37, against 1,139 of the wavefront).
+        Renderer m(scene, wf::GpuMode::Megakernel);
+        m.set_camera(cam, width, height);
+        apply_tuning(m, best);
+        mk_ms = measure(m, pw) * samples / samples_w;
     }
     best.megakernel_msamples_s = samples / mk_ms / 1e3;
     if (try_wavefront) best.wavefront_msamples_s = samples / wf_ms / 1e3;
