@@ -111,7 +111,7 @@ void BatchLauncher::launch(const std::vector<JobSpec>& jobs, const std::vector<J
         wide_nodes = std::max(wide_nodes, desc[i].s.n_nodes);
     }
     if (!all_wide) wide_nodes = 0;
-    const int tree = wide_nodes == 0 ? 0 : wide_nodes < kSmallTree ? 1 : 2;  // what of it the launch depends on
+    const int tree = wide_nodes == 0 ? 0 : wide_nodes < kSmallTreeMega ? 1 : 2;  // what of it a captured launch depends on
     if (wf_) {
         last_launches_ = wf_->run_batch(d_jobs_, d_hdr_, d_counters_, count_rays, wide_nodes, stream);
         launch_film_commit_jobs(d_jobs_, d_hdr_, max_jobs_, stream);

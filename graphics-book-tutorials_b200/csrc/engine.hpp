@@ -142,7 +142,7 @@ struct MegakernelConfig {
 };
 // `cfg` with its defaults filled in. wide_nodes: 0 for the preorder kernel, else the launch takes the ordered traversal over
 // trees of at most that many preorder nodes.
-constexpr int kSmallTree = 4096;
+constexpr int kSmallTreeMega = 256;
 MegakernelConfig with_defaults(const MegakernelConfig& cfg, int wide_nodes);
 // Split mode keeps each path's radiance (3 floats) per (pixel, sample) until the ordered commit;
 // automatic splitting keeps that buffer under kSplitBufferBytes (renders above it run in sub-passes).
@@ -244,11 +244,15 @@ struct WavefrontConfig {
     int leaf_batch = 0;       // a warp tests primitives once this many lanes hold a pending leaf; 0: the default
     bool speculate = true;    // as in MegakernelConfig
 };
-// The defaults for the preorder steps, the ordered traversal, and the ordered traversal over a small tree (kSmallTree). Ordered
+// The defaults for the preorder steps, the ordered traversal, and the ordered traversal over a small tree (kSmallTreeWavefront). Ordered
 // rays are fetched again sooner than they would trace on with few lanes (icospheres 1280x720x16 at 4 / 8 / 12 / 16 lanes: 13.68 /
 // 13.28 / 13.32 / 13.59 ms), and the 64-register form is the faster one (8 / 6 CTAs: 13.3 / 13.5 ms, heightfield 9.2 / 9.8; 10 CTAs
 // lost 9% and 6% when the phases were four). Over a small tree the barriers count more than the latency of the nodes
 // (cornell36 320x180x16: 8 / 6 CTAs 1.01 / 0.87 ms) and the end of a phase more than its lanes (8 / 4 lanes: 0.87 / 0.85 ms).
+// The line between them, over bumpy sheets and triangle soups of growing size in the Cornell box (640x360x16, 6 CTAs and 4 lanes
+// against 8 and 8): 3.53 / 3.69 ms at 525 nodes, 3.68 / 3.68 at 2,461, 5.08 / 5.13 at 4,137, 4.00 / 3.95 at 4,895, 5.88 / 5.85 at
+// 8,143, 12.5 / 12.0 at 262,191.
+constexpr int kSmallTreeWavefront = 4096;
 constexpr int kWfOccupancy[3] = {10, 8, 6}, kWfMinActive[3] = {24, 8, 4}, kWfLeafBatch[3] = {8, 16, 16};
 
 // Launch configuration of a batch or a server: the arm and its knobs.

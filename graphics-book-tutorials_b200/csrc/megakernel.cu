@@ -439,12 +439,14 @@ MegakernelConfig with_defaults(const MegakernelConfig& cfg, int wide_nodes) {
     MegakernelConfig c = cfg;
     const bool wide = wide_nodes > 0;
     if (c.occupancy < 0) c.occupancy = 10;
-    // Ordered traversal: a ray through a tree of a few thousand nodes is short next to shading, which then waits for
-    // more lanes (cornell36 320x180x16, min_active 4 / 8: 0.642 / 0.673 ms); a longer one is not (icospheres
-    // 1280x720x16: 13.3 / 13.0 ms, heightfield 8.74 / 8.50).
+    // Ordered traversal: a ray through a tree of a few dozen nodes is short next to shading, which then waits for
+    // more lanes (cornell36, 47 nodes, 320x180x16, min_active 4 / 8: 0.642 / 0.673 ms); a longer one is not (icospheres
+    // 1280x720x16: 13.3 / 13.0 ms, heightfield 8.74 / 8.50). In between, bumpy sheets and triangle soups in the Cornell box
+    // (640x360x16): 2.40 / 2.42 ms at 63 nodes, 2.36 / 2.36 at 95, 2.86 / 2.84 at 143, 3.14 / 3.03 at 337, 3.52 / 3.35 at
+    // 1,253, 5.00 / 4.77 at 4,137, 4.19 / 3.86 at 9,651.
     // Preorder batches (many jobs of several scenes) traverse best with a lower min_active than one render of one
     // scene: on the 64-job mix on a B200, 12 took 1,168 ms against 1,206 at 16.
-    if (c.min_active <= 0) c.min_active = wide ? (wide_nodes < kSmallTree ? 4 : 8) : cfg.batch ? 12 : 16;
+    if (c.min_active <= 0) c.min_active = wide ? (wide_nodes < kSmallTreeMega ? 4 : 8) : cfg.batch ? 12 : 16;
     // A primitive round costs as much as a node round, so it waits for more lanes than in preorder (16 / 24: icospheres
     // 13.9 / 13.8 ms).
     if (c.leaf_batch <= 0) c.leaf_batch = wide ? 24 : 12;

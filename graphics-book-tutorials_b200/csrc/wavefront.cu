@@ -1138,7 +1138,7 @@ int WavefrontEngine::run(const DevScene& s, const DevFilm& film, DevCounters* co
                          wf::StageTimes* stages, cudaStream_t stream, KernelTimer* timer) {
     if (p.sample_count <= 0 || film.pixels <= 0) return 0;
     State& st = *state_;
-    const int w = !cfg_.speculate || !wide_usable(s) ? 0 : s.n_nodes < kSmallTree ? 2 : 1;
+    const int w = !cfg_.speculate || !wide_usable(s) ? 0 : s.n_nodes < kSmallTreeWavefront ? 2 : 1;
     const int chunks = chunks_for(film.pixels, p.sample_count);
     WfArgs a{};
     a.job0 = make_job(s, film, nullptr, p.first_sample, p.sample_count, chunks, p.seed, p.max_depth);
@@ -1187,7 +1187,7 @@ int WavefrontEngine::run(const DevScene& s, const DevFilm& film, DevCounters* co
 int WavefrontEngine::run_batch(const JobDesc* d_jobs, const BatchHeader* d_hdr, DevCounters* counters,
                                bool count_rays, int wide_nodes, cudaStream_t stream) {
     reserve_direct();  // a batch may hold direct-mode jobs
-    const int w = !cfg_.speculate || wide_nodes == 0 ? 0 : wide_nodes < kSmallTree ? 2 : 1;
+    const int w = !cfg_.speculate || wide_nodes == 0 ? 0 : wide_nodes < kSmallTreeWavefront ? 2 : 1;
     WfArgs a{};
     a.jobs = d_jobs;
     a.hdr = d_hdr;
