@@ -225,22 +225,6 @@ std::vector<float4> host_wide(const std::vector<float4>& nodes, int nn, std::vec
     return wide;
 }
 
-struct HostStack {
-    int code[kStackShared + kStackLocal];
-    void push(WideState& s, int c) {
-        if (s.sp == kStackShared + kStackLocal) s.redo |= kRedoRay;
-        else code[s.sp++] = c;
-    }
-    void push3(WideState& s, int a, bool pa, int b, bool pb, int c, bool pc) {
-        if (pa) push(s, a);
-        if (pb) push(s, b);
-        if (pc) push(s, c);
-    }
-    void pop(WideState& s) const {
-        if (s.sp > 0) s.cur = code[--s.sp];
-    }
-};
-
 }  // namespace
 
 void traverse_ordered_check(const wf::Scene& host, const float* rays, int n, bool anyhit, float* hits,
@@ -258,7 +242,10 @@ void traverse_ordered_check(const wf::Scene& host, const float* rays, int n, boo
     if (check_boxes_nested(host.nodes)) wide = host_wide(nodes, nn, prims, ns);
     for (int k = 0; k < 4; ++k) counts[k] = 0;
     counts[3] = (long long)(wide.size() / kWideFloat4);
-    HostStack stack;
+    // the kernels' lane stack, the last column of four
+    constexpr int kColumns = 4, kColumn = 3;
+    int stack_words[kStackShared * kColumns], stack_deep[kStackLocal];
+    LaneStack<kColumns> stack{stack_words, stack_deep};
     for (int k = 0; k < n; ++k) {
         const float* r = rays + 8 * (size_t)k;
         const wf::Vec3 o{r[0], r[1], r[2]}, d{r[4], r[5], r[6]};
@@ -270,7 +257,7 @@ void traverse_ordered_check(const wf::Scene& host, const float* rays, int n, boo
         h.u = h.v = 0.0f;
         bool redo = wide.empty();
         if (!redo) {
-            wide_begin(d, r[7], true, 0, &ray, &s);
+            wide_begin(d, r[7], true, kColumn, &ray, &s);
             while (s.cur != 0 || s.pend != 0) {
                 if (s.pend != 0) {
                     ++counts[1];

@@ -154,7 +154,7 @@ int launch_wide_build(const DevScene& s, float4* prims, int n_prims, float4* wid
         if (levels <= 0) levels = std::max(1, (int)std::ceil(0.62 * std::log2((double)capacity)) - 2);
     }
     if (first_level > 0 && levels <= 0) levels = 8;
-    const int grid = std::min((capacity + 63) / 64, 148 * 16);
+    const int grid = std::min((capacity + 63) / 64, 148 * 16);  // 148 SMs, 16 CTAs each: a level strides over the rest
     for (int l = first_level; l < first_level + levels; ++l)
         wide_build_level<<<grid, 64, 0, stream>>>(s.nodes, s.n_nodes, wide, capacity, empty, l, ctl);
     cuda_check(cudaGetLastError(), "wide build launch");

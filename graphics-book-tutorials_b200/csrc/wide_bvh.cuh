@@ -52,7 +52,8 @@ constexpr float kInvMax = 1.099511627776e12f;    // 2^40, as for coordinates: no
 constexpr float kCoordMax = 1.099511627776e12f;
 
 // A wide node is 4 float4 (64 B, two 32-byte loads): a grid (origin, step per axis) and the planes of up to 4 child
-// boxes on it, 8 bits each, child k's in byte k:
+// boxes on it, 8 bits each (after Ylitie, Karras and Laine, "Efficient Incoherent Ray Traversal on GPUs Through Compressed Wide
+// BVHs", HPG 2017, whose nodes have 8 children), child k's in byte k:
 //   {origin.x, origin.y, step.x, step.y} {origin.z, step.z, lo.x[4], hi.x[4]}
 //   {lo.y[4], hi.y[4], lo.z[4], hi.z[4]} {code}[4]
 // (the steps stored times 2^15, see plane_of)
@@ -107,6 +108,39 @@ WF_HD void wide_begin(wf::Vec3 d, float tmax, bool has_nodes, int stack_base, Tr
     s->best = tmax;
     s->redo = fit ? 0 : kRedoRay;
 }
+
+// A lane's stack of nodes, one column per thread, so that lanes at different depths never meet in a bank: the first
+// entries in shared memory (WideState::sp is the word index there), deeper ones in local memory.
+template <int BLOCK>
+struct LaneStack {
+    int* words;  // kStackShared * BLOCK words, shared
+    int* deep;   // kStackLocal words, local
+    WF_HD void push3(WideState& s, int a, bool pa, int b, bool pb, int c, bool pc) {
+        if (s.sp < (kStackShared - 2) * BLOCK) {  // room for three
+            if (pa) { words[s.sp] = a; s.sp += BLOCK; }
+            if (pb) { words[s.sp] = b; s.sp += BLOCK; }
+            if (pc) { words[s.sp] = c; s.sp += BLOCK; }
+        } else {
+            if (pa) push_deep(s, a);
+            if (pb) push_deep(s, b);
+            if (pc) push_deep(s, c);
+        }
+    }
+    WF_HD void push_deep(WideState& s, int code) {
+        if (s.sp < kStackShared * BLOCK) words[s.sp] = code;
+        else if (s.sp < (kStackShared + kStackLocal) * BLOCK) deep[(s.sp - s.base) / BLOCK - kStackShared] = code;
+        else {
+            s.redo |= kRedoRay;
+            return;
+        }
+        s.sp += BLOCK;
+    }
+    WF_HD void pop(WideState& s) const {
+        if (s.sp == s.base) return;
+        s.sp -= BLOCK;
+        s.cur = s.sp < kStackShared * BLOCK ? words[s.sp] : deep[(s.sp - s.base) / BLOCK - kStackShared];
+    }
+};
 
 // The lane's next node: `cur` stays while it is usable; a leaf becomes the pending one when none is; an
 // empty `cur` is refilled from the stack.
