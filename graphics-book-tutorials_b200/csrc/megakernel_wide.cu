@@ -5,11 +5,11 @@
 // leaves open. What differs, and what it is worth (B200,
 // icospheres / heightfield 1280x720x16, cornell36 320x180x16; the preorder kernel takes 22.9 / 12.3 / 0.82 ms):
 //
-//  * Instruction issue bounds it (0.70 of the slots, 15.5 lanes per instruction; DRAM idle): a warp executes about 800
-//    instructions per sample of its lanes, 40% of them in node steps. So the node step is short (two 32-byte loads,
+//  * Instruction issue bounds it (0.76 of the slots, 15.5 lanes per instruction; DRAM idle): about 790 warp instructions
+//    are executed per sample, 40% of them in node steps. So the node step is short (two 32-byte loads,
 //    packed multiply-adds, one byte permute per plane, a stack in shared memory): 15.3 -> 14.4 ms against the
 //    straightforward form.
-//  * The instruction cache comes next (1.6 of 11 stall cycles per issue): rays start, paths start and scattering
+//  * The instruction cache came next (1.6 stall cycles per issue; 0.6 now): rays start, paths start and scattering
 //    events end at one place each in the code, whatever the lane's material or the reason; cosine and sine are
 //    one out-of-line copy. 14.4 / 8.9 / 0.69 -> 13.0 / 8.5 / 0.64 ms. (Path state in a pool of 64 contexts per warp, so
 //    that 18 lanes are active per instruction, was slower, 16.2 ms: the pool's bookkeeping and shared memory
