@@ -9,6 +9,7 @@
 #include <cstring>
 #include <numeric>
 #include "batch.hpp"
+#include "counts.hpp"
 #include "../../include/wfb200.h"
 
 namespace wfb {
@@ -103,7 +104,7 @@ void BatchLauncher::launch(const std::vector<JobSpec>& jobs, const std::vector<J
                "upload job table");
     cuda_check(cudaEventRecord(staged_, stream), "cudaEventRecord");
     cuda_check(cudaMemsetAsync(d_counters_, 0, sizeof(DevCounters), stream), "zero counters");
-    bool all_split = n > 0, all_wide = n > 0;
+    bool all_split = n > 0, all_wide = n > 0 && (wf_ || units <= kMaxWideUnits);
     int wide_nodes = 0;
     for (int i = 0; i < n; ++i) {
         all_split = all_split && desc[i].chunks > 1;

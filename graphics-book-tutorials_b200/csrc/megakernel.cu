@@ -39,6 +39,7 @@
 //  * Ray counters live in registers and are folded with one atomic per warp at exit.
 #include <algorithm>
 #include <type_traits>
+#include "counts.hpp"
 #include "engine.hpp"
 #include "../../include/wfb200.h"
 
@@ -491,7 +492,8 @@ JobDesc make_job(const DevScene& s, const DevFilm& film, float* lbuf, int first_
 int launch_megakernel(const DevScene& s, const DevFilm& film, DevCounters* counters, unsigned int* work_counter,
                       float* lbuf, const PassParams& p, const MegakernelConfig& config, int chunks,
                       cudaStream_t stream, KernelTimer* timer, bool work_is_zero) {
-    const bool wide = config.speculate && !p.count_rays && wide_usable(s);
+    const bool wide = config.speculate && !p.count_rays && wide_usable(s) &&
+                      (unsigned long long)film.pixels * (unsigned)std::max(1, chunks) <= kMaxWideUnits;
     const MegakernelConfig cfg = with_defaults(config, wide ? s.n_nodes : 0);
     if (p.sample_count <= 0 || film.pixels <= 0) return 0;
     if (chunks > 1 && lbuf == nullptr) throw Error(WFB_ERR_INTERNAL, "split megakernel needs a sample buffer");

@@ -77,7 +77,7 @@ __global__ void __launch_bounds__(kBlock, kCtas) megakernel_wide(const WideArgs 
     // sooner than one of 32 that diverge.
     const unsigned share = warp_share(total_units, gridDim.x * (kBlock / 32));
     bool out_of_work = (unsigned)lane >= share;
-    const int min_active = spread_min_active(a.min_active, share);
+    const int min_active = min(a.min_active, (int)min((share + 1) / 2, 32u));
     wf::Vec3 o{0.f, 0.f, 0.f};
     TravRay ray;
     ray.d = ray.inv_d = wf::Vec3{0.f, 0.f, 0.f};

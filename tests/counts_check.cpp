@@ -19,19 +19,12 @@ int main() {
             for (long long n = mid - 3; n <= mid + 3; ++n)
                 if (n >= 1 && n <= 0x7fffffffll)
                     want(wfb::scan_tile_count((int)n, tile), (n + tile - 1) / tile, "scan_tile_count", n, tile);
-    // units near 0 and the end of the range; warps of one CTA, of small grids, and of 148 SMs with 8 CTAs of 4 warps
-    for (long long warps : {4ll, 32ll, 1000ll, 148ll * 8 * 4})
-        for (long long mid : {0ll, 5000ll, 1ll << 31, 0xffffffffll - 4736, 0xfffffffell})
-            for (long long u = mid - 3; u <= mid + 3; ++u)
-                if (u >= 0 && u <= 0xffffffffll) {
-                    const long long share = (u + warps - 1) / warps;
-                    want(wfb::warp_share((unsigned)u, (unsigned)warps), share, "warp_share", u, warps);
-                    for (int least : {1, 4, 8, 16, 32}) {
-                        const long long half = (share + 1) / 2;
-                        want(wfb::spread_min_active(least, (unsigned)share), half < least ? half : least, "spread_min_active",
-                             least, share);
-                    }
-                }
+    // units near 0 and up to the largest launch; warps of one CTA, of small grids, of 148 SMs with 8 CTAs of 4 warps, and the most
+    for (long long warps : {4ll, 32ll, 1000ll, 148ll * 8 * 4, 65536ll})
+        for (long long mid : {0ll, 5000ll, 1ll << 31, 0xffffffffll - 70000, (long long)wfb::kMaxWideUnits})
+            for (long long u = mid - 3; u <= mid; ++u)
+                if (u >= 0)
+                    want(wfb::warp_share((unsigned)u, (unsigned)warps), (u + warps - 1) / warps, "warp_share", u, warps);
     std::printf("ok %lld\n", checks);
     return 0;
 }

@@ -1,5 +1,5 @@
 """Tile and share counts at the ends of their ranges (csrc/counts.hpp) on the CPU: arrays of up to 2^31 - 1 elements
-and launches of up to 2^32 - 2 work units (tests/counts_check.cpp)."""
+and launches of up to 2^32 - 2^16 work units (tests/counts_check.cpp)."""
 import os
 import shutil
 import subprocess
